@@ -4,20 +4,20 @@
 //   host    k-vectors of the cell inside the k_cutoff ball (one of each +-k
 //           pair), the density's Fourier transform f(k) and the radial
 //           integral R_nl(|k|) (spline or analytic) per k-vector
-//   kernel  lode_projection_kernel: T[k][lm][n] = R_nl(|k|) Y_lm(k^)
+//   kernel  lode_projection_kernel: T[k][(l m n)] = R_nl(|k|) Y_lm(k^), the
+//           even l first, then the odd l
 //   kernel  lode_phases_kernel: cos(k.r_i), sin(k.r_i) for every atom and k
 //   kernel  lode_type_sums_kernel: the same summed over the atoms of each type
-//   kernel  lode_values_kernel: one CTA per (centre, neighbour type), every
-//           thread a few (l, m, n) coefficients, sum over k of
-//           4 pi / V f(k) S_i^t(k) T[k][lm][n] with the structure factor
-//           S_i^t (real part for even l, imaginary for odd l)
-//   kernel  lode_gradients_kernel: one CTA per gradient row (centre i,
-//           atom j, neighbour type t), the pair factor of (i, j) against the
-//           same table times the k-vector
+//   kernel  lode_gemm_kernel: values (rows: centre i towards neighbour type t)
+//           and positions gradients (rows: centre i, atom j, neighbour type
+//           t, component x) as products [rows][k] x T[k][(l m n)] on the FP64
+//           tensor cores, with the structure factor S_i^t(k) or the pair
+//           factor of (i, j), times 4 pi / V f(k), made on the way into
+//           shared memory
 //
-// Every coefficient is summed over k in featomic's order with featomic's
-// expressions (the sign (-1)^{l/2}, (-1)^{(l+1)/2} applied at the end, which
-// is exact), then the central-atom and k = 0 terms in featomic's order.
+// The sums over k run in featomic's order inside each split of the k-vectors
+// (the sign (-1)^{l/2}, (-1)^{(l+1)/2} applied at the end, which is exact),
+// then the central-atom and k = 0 terms in featomic's order.
 #include <algorithm>
 #include <chrono>
 #include <cmath>
@@ -326,274 +326,418 @@ namespace fb200 {
 namespace {
 
 constexpr int LODE_LCAP = 16;
-constexpr int LODE_CHUNK = 128;  // k-vectors staged in shared memory at a time
-constexpr int LODE_GROUP = 8;    // centres of one neighbour type per values CTA
+constexpr int LODE_KB = 16;       // k-vectors per step of the product, and the padding of their number
+constexpr int LODE_ROWS = 64;     // rows of one tile of the product
 constexpr int LODE_THREADS = 128;
-constexpr int LODE_Q = 4;        // coefficients per thread
+constexpr int LODE_LDA = LODE_KB + 4;  // pitch = 4 (mod 16) doubles: fragment loads hit every bank once
 
-__host__ __device__ inline int l_of(int lm) {
-    int l = 0;
-    while ((l + 1) * (l + 1) <= lm) l++;
-    return l;
-}
-
-// T[k][lm N + n] = R_nl(|k|) Y_lm(k^) (spherical_expansion.rs:226-274):
-// one thread per k-vector
-__global__ void lode_projection_kernel(int K, int L, int N, const double* __restrict__ dir,
-                                       const double* __restrict__ radial, DeviceYlm ylm, double* __restrict__ T) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= K) return;
-    double Y[(LODE_LCAP + 1) * (LODE_LCAP + 1)];
-    ylm_compute<double, LODE_LCAP>(ylm, dir[3 * k], dir[3 * k + 1], dir[3 * k + 2], Y, nullptr, nullptr, nullptr);
-    const int L2 = (L + 1) * (L + 1);
-    double* out = T + (size_t)k * L2 * N;
-    for (int lm = 0; lm < L2; lm++) {
-        const int l = l_of(lm);
-        const double* R = radial + ((size_t)k * (L + 1) + l) * N;
-        for (int n = 0; n < N; n++) out[lm * N + n] = R[n] * Y[lm];
-    }
-}
-
-// cos and sin of k.r for every (atom, k) (spherical_expansion.rs:92-111),
-// k.r = (|k| k^) . r in featomic's order
-__global__ void lode_phases_kernel(int n_atoms, int K, const double* __restrict__ positions,
-                                   const double* __restrict__ kvec, double* __restrict__ C, double* __restrict__ S) {
-    const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= (int64_t)n_atoms * K) return;
-    const int i = (int)(idx / K), k = (int)(idx - (int64_t)i * K);
-    const double* p = positions + 3 * i;
-    const double* q = kvec + 3 * k;
-    const double s = q[0] * p[0] + q[1] * p[1] + q[2] * p[2];
-    double sn, cs;
-    sincos(s, &sn, &cs);
-    C[idx] = cs;
-    S[idx] = sn;
-}
-
-// sum of cos(k.r_j), sin(k.r_j) over the atoms j of each type, in atom order
-// (spherical_expansion.rs:125-141)
-__global__ void lode_type_sums_kernel(int n_atoms, int K, int n_species, const int32_t* __restrict__ species,
-                                      const double* __restrict__ C, const double* __restrict__ S,
-                                      double* __restrict__ Ct, double* __restrict__ St) {
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= n_species * K) return;
-    const int t = idx / K, k = idx - t * K;
-    double sc = 0.0, ss = 0.0;
-    for (int j = 0; j < n_atoms; j++) {
-        if (species[j] != t) continue;
-        sc += C[(size_t)j * K + k];
-        ss += S[(size_t)j * K + k];
-    }
-    Ct[idx] = sc;
-    St[idx] = ss;
-}
-
-struct LodeArgs {
-    int n_atoms, K, S, L, N;
-    const int32_t* species;     // [n_atoms] species index of the system's atoms
-    const double *C, *Sn;       // [n_atoms][K]
-    const double *Ct, *St;      // [S][K]
-    const double* gdf;          // [K] 4 pi / V f(k)
-    const double* T;            // [K][(L + 1)^2][N]
-    const double* kvec;         // [K][3] |k| k^ (unused by the values)
-    const double* knorm;        // [K]
-    const double* kdir;         // [K][3]
-    // values
-    const int32_t* row;         // [n_atoms][S] sample row of atom i in the blocks (type_i, t), -1: none
-    const int64_t* off_values;  // [S][S][L + 1] offset of each block's values
-    const int32_t* type_count;  // [S] atoms of each type in the system
-    const double* center;       // [N] central-atom contribution
-    const double* k0;           // [N] 4 pi / V times the k = 0 term
-    double center_factor;       // 1 - center_atom_weight
-    int add_k0;
-    // gradients
-    const int32_t* tasks;       // [n_tasks][4] (i, j, t, row)
-    const int64_t* off_positions;
-    double* out;
+// Columns of T and of the product: the even l, then (from `odd0`) the odd l,
+// each in (l, m, n) order and padded to 16 bytes
+struct LodeColumns {
+    int n_even, n_odd, odd0, ld;
 };
+
+LodeColumns lode_columns(int L, int N) {
+    LodeColumns c{};
+    for (int l = 0; l <= L; l++) (l & 1 ? c.n_odd : c.n_even) += (2 * l + 1) * N;
+    c.odd0 = (c.n_even + 1) & ~1;
+    c.ld = c.odd0 + ((c.n_odd + 1) & ~1);
+    return c;
+}
+
+// (l, m) rows of one parity before channel l: sum of 2 l' + 1 over l' = l - 2, l - 4, ...
+__host__ __device__ inline int lode_lm_before(int l) { return l * (l - 1) / 2; }
 
 __device__ inline double lode_phase(int l) {
     // spherical_expansion.rs:667-671
     return (l % 2 == 0) ? ((l / 2) % 2 == 0 ? 1.0 : -1.0) : (((l + 1) / 2) % 2 == 0 ? 1.0 : -1.0);
 }
 
-// values (spherical_expansion.rs:616-723): CTA (neighbour type t, group of
-// LODE_GROUP centres of one type, tile of coefficients); each thread sums
-// LODE_Q coefficients of every centre of the group over k
-__global__ void __launch_bounds__(LODE_THREADS) lode_values_kernel(LodeArgs a, const int32_t* __restrict__ groups,
-                                                                    int n_groups) {
-    const int t = blockIdx.x % a.S;
-    const int g = blockIdx.x / a.S;
-    if (g >= n_groups) return;
-    const int32_t* centres = groups + (size_t)g * LODE_GROUP;  // -1 padded, all of one type
-    const int L2 = (a.L + 1) * (a.L + 1), outs = L2 * a.N;
-    const int o0 = blockIdx.y * LODE_THREADS * LODE_Q;
-    __shared__ double wr[LODE_GROUP][LODE_CHUNK], wi[LODE_GROUP][LODE_CHUNK];
-    double acc[LODE_GROUP][LODE_Q];
-#pragma unroll
-    for (int c = 0; c < LODE_GROUP; c++)
-#pragma unroll
-        for (int q = 0; q < LODE_Q; q++) acc[c][q] = 0.0;
-    int parity[LODE_Q];
-#pragma unroll
-    for (int q = 0; q < LODE_Q; q++) {
-        const int o = o0 + q * LODE_THREADS + threadIdx.x;
-        parity[q] = o < outs ? (l_of(o / a.N) & 1) : 0;
-    }
-    for (int k0 = 0; k0 < a.K; k0 += LODE_CHUNK) {
-        const int nk = min(LODE_CHUNK, a.K - k0);
-        __syncthreads();
-        for (int w = threadIdx.x; w < LODE_GROUP * nk; w += blockDim.x) {
-            const int c = w / nk, kk = w - c * nk, k = k0 + kk;
-            const int i = centres[c];
-            if (i < 0 || a.row[(size_t)i * a.S + t] < 0) {
-                wr[c][kk] = 0.0;
-                wi[c][kk] = 0.0;
-                continue;
-            }
-            const double ci = a.C[(size_t)i * a.K + k], si = a.Sn[(size_t)i * a.K + k];
-            const double ct = a.Ct[(size_t)t * a.K + k], st = a.St[(size_t)t * a.K + k];
-            // structure factor per centre (:143-155), real and imaginary part
-            const double real = 2.0 * (ci * ct + si * st);
-            const double imag = 2.0 * (si * ct - ci * st);
-            wr[c][kk] = a.gdf[k] * real;
-            wi[c][kk] = a.gdf[k] * imag;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int q = 0; q < LODE_Q; q++) {
-            const int o = o0 + q * LODE_THREADS + threadIdx.x;
-            if (o >= outs) continue;
-            const double* Tk = a.T + (size_t)k0 * outs + o;
-            const double(*w)[LODE_CHUNK] = parity[q] ? wi : wr;
-            int kk = 0;
-            // four k-vectors per step: the loads first, then each sum in k order
-            for (; kk + 4 <= nk; kk += 4) {
-                double tv[4];
-#pragma unroll
-                for (int u = 0; u < 4; u++) tv[u] = Tk[(size_t)(kk + u) * outs];
-#pragma unroll
-                for (int u = 0; u < 4; u++)
-#pragma unroll
-                    for (int c = 0; c < LODE_GROUP; c++) acc[c][q] += w[c][kk + u] * tv[u];
-            }
-            for (; kk < nk; kk++) {
-                const double tv = Tk[(size_t)kk * outs];
-#pragma unroll
-                for (int c = 0; c < LODE_GROUP; c++) acc[c][q] += w[c][kk] * tv;
-            }
+// T[k][column] = R_nl(|k|) Y_lm(k^) (spherical_expansion.rs:226-274) for `kc`
+// k-vectors per CTA, zero for the padding of their number: a thread per (k, m)
+// for the Legendre columns and harmonics, a thread per (k, l) for the spline
+// of the radial integral (`radial` holds it when there is no spline), then
+// every thread writes columns.  One thread per k-vector, as it was, left the
+// chip to 36 CTAs and the radial integrals to the host: 65 us for 4522
+// k-vectors, and 14 us now, with 2 MB less to copy up.
+__global__ void __launch_bounds__(128) lode_projection_kernel(int K, int Kp, int kc, int N, LodeColumns cols,
+                                                              const double* __restrict__ dir,
+                                                              const double* __restrict__ norm,
+                                                              const double* __restrict__ radial, DeviceRadial spline,
+                                                              DeviceYlm ylm, double* __restrict__ T) {
+    extern __shared__ double proj_smem[];
+    const int L = ylm.lmax, L1 = L + 1, L2 = L1 * L1, NP = L1 * (L + 2) / 2;
+    double* P = proj_smem;               // [kc][NP]
+    double* Y = P + kc * NP;             // [kc][L2]
+    double* R = Y + kc * L2;             // [kc][L1][N]
+    const int k0 = blockIdx.x * kc;
+    for (int w = threadIdx.x; w < 2 * kc * L1; w += blockDim.x) {
+        const bool column = w < kc * L1;
+        const int v = column ? w : w - kc * L1;
+        const int q = v / L1, j = v - q * L1, k = k0 + q;
+        if (k >= K) continue;
+        if (column) {
+            ylm_legendre_column(ylm, ylm_angles(dir[3 * k], dir[3 * k + 1], dir[3 * k + 2]), j, P + q * NP);
+        } else if (radial == nullptr) {
+            radial_spline_compute(spline, j, norm[k], R + (q * L1 + j) * N, nullptr);
+        } else {
+            for (int n = 0; n < N; n++) R[(q * L1 + j) * N + n] = radial[((size_t)k * L1 + j) * N + n];
         }
     }
-#pragma unroll
-    for (int q = 0; q < LODE_Q; q++) {
-        const int o = o0 + q * LODE_THREADS + threadIdx.x;
-        if (o >= outs) continue;
-        const int lm = o / a.N, n = o - lm * a.N, l = l_of(lm), mi = lm - l * l;
-        const double phase = lode_phase(l);
-#pragma unroll
-        for (int c = 0; c < LODE_GROUP; c++) {
-            const int i = centres[c];
-            if (i < 0) continue;
-            const int r = a.row[(size_t)i * a.S + t];
-            if (r < 0) continue;
-            const int ti = a.species[i];
-            double x = 0.0;
-            if (l == 0) {
-                // central atom (:378-426), then the k = 0 term once per atom
-                // of type t (:635-661)
-                if (t == ti) x -= a.center_factor * a.center[n];
-                if (a.add_k0)
-                    for (int j = 0; j < a.type_count[t]; j++) x += a.k0[n];
-            }
-            x += phase * acc[c][q];
-            const int64_t off = a.off_values[((size_t)ti * a.S + t) * (a.L + 1) + l];
-            a.out[off + ((int64_t)r * (2 * l + 1) + mi) * a.N + n] = x;
+    __syncthreads();
+    for (int w = threadIdx.x; w < kc * L1; w += blockDim.x) {
+        const int q = w / L1, m = w - q * L1, k = k0 + q;
+        if (k >= K) continue;
+        ylm_column_outputs(ylm, ylm_angles(dir[3 * k], dir[3 * k + 1], dir[3 * k + 2]), m, P + q * NP, Y + q * L2,
+                           (double*)nullptr, (double*)nullptr, (double*)nullptr);
+    }
+    __syncthreads();
+    for (int c = threadIdx.x; c < cols.ld; c += blockDim.x) {
+        const bool odd = c >= cols.odd0;
+        const int pos = odd ? c - cols.odd0 : c;
+        const bool pad = pos >= (odd ? cols.n_odd : cols.n_even);
+        const int row = pos / N, n = pos - row * N;
+        int l = odd ? 1 : 0;
+        while (lode_lm_before(l + 2) <= row) l += 2;
+        const int lm = l * l + row - lode_lm_before(l);
+        for (int q = 0; q < kc; q++) {
+            const int k = k0 + q;
+            if (k >= Kp) break;
+            T[(size_t)k * cols.ld + c] = (pad || k >= K) ? 0.0 : R[(q * L1 + l) * N + n] * Y[q * L2 + lm];
         }
     }
 }
 
-// positions gradients (spherical_expansion.rs:725-873): CTA (gradient row,
-// tile of coefficients); the pair factor of (i, j) per k staged in shared
-// memory with |k| and k^
-__global__ void __launch_bounds__(LODE_THREADS) lode_gradients_kernel(LodeArgs a, int n_tasks) {
-    const int task = blockIdx.x;
-    if (task >= n_tasks) return;
-    const int i = a.tasks[4 * task], j = a.tasks[4 * task + 1], t = a.tasks[4 * task + 2], r = a.tasks[4 * task + 3];
-    const int ti = a.species[i];
-    const int L2 = (a.L + 1) * (a.L + 1), outs = L2 * a.N;
-    const int o0 = blockIdx.y * LODE_THREADS * LODE_Q;
-    __shared__ double pe[LODE_CHUNK], po[LODE_CHUNK], kn[LODE_CHUNK], kd[LODE_CHUNK][3];
-    double acc[LODE_Q][3];
+// cos and sin of k.r for every (atom, k) (spherical_expansion.rs:92-111),
+// k.r = (|k| k^) . r in featomic's order; zero for the padding of k
+__global__ void lode_phases_kernel(int n_atoms, int K, int Kp, const double* __restrict__ positions,
+                                   const double* __restrict__ kvec, double* __restrict__ C, double* __restrict__ S) {
+    const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx >= (int64_t)n_atoms * Kp) return;
+    const int i = (int)(idx / Kp), k = (int)(idx - (int64_t)i * Kp);
+    double sn = 0.0, cs = 0.0;
+    if (k < K) {
+        const double* p = positions + 3 * i;
+        const double* q = kvec + 3 * k;
+        sincos(q[0] * p[0] + q[1] * p[1] + q[2] * p[2], &sn, &cs);
+    }
+    C[idx] = cs;
+    S[idx] = sn;
+}
+
+// 4 pi / V f(k) times the sums of cos(k.r_j), sin(k.r_j) over the atoms j of
+// each type (spherical_expansion.rs:125-141), from the atoms sorted by type:
+// CTA (32 k-vectors, type) with eight atoms in flight per k-vector, added in
+// a fixed order.  (A thread per (type, k) that walked over every atom took
+// 134 us for 1000 atoms and 4522 k-vectors, this takes 13 us.)
+__global__ void __launch_bounds__(256) lode_type_sums_kernel(int K, int Kp, const int32_t* __restrict__ sorted_atoms,
+                                                             const int32_t* __restrict__ type_start,
+                                                             const double* __restrict__ gdf,
+                                                             const double* __restrict__ C, const double* __restrict__ S,
+                                                             double* __restrict__ Ct, double* __restrict__ St) {
+    __shared__ double part[2][8][32];
+    const int x = threadIdx.x & 31, y = threadIdx.x >> 5, t = blockIdx.y;
+    const int k = blockIdx.x * 32 + x;
+    double sc = 0.0, ss = 0.0;
+    if (k < K) {
+        for (int q = type_start[t] + y; q < type_start[t + 1]; q += 8) {
+            const size_t at = (size_t)sorted_atoms[q] * Kp + k;
+            sc += C[at];
+            ss += S[at];
+        }
+    }
+    part[0][y][x] = sc;
+    part[1][y][x] = ss;
+    __syncthreads();
+    if (y >= 2 || k >= Kp) return;
+    double sum = 0.0;
+    for (int q = 0; q < 8; q++) sum += part[y][q][x];
+    (y == 0 ? Ct : St)[(size_t)t * Kp + k] = k < K ? gdf[k] * sum : 0.0;
+}
+
+struct LodeArgs {
+    int Kp, S, L, N;            // Kp: k-vectors padded to LODE_KB
+    LodeColumns cols;
+    const int32_t* species;     // [n_atoms] species index of the system's atoms
+    const double *C, *Sn;       // [n_atoms][Kp]
+    const double *Ct, *St;      // [S][Kp] sums over the atoms of a type, times 4 pi / V f(k)
+    const double* gdf;          // [Kp] 4 pi / V f(k), zero in the padding
+    const double* T;            // [Kp][ld]
+    const double* kvec;         // [Kp][3] |k| k^
+    // values: rows are the atoms, for each type in `present`
+    const int32_t* present;     // [n_present] types of the system
+    const int32_t* row;         // [n_atoms][S] sample row of atom i in the blocks (type_i, t)
+    const int64_t* off_values;  // [S][S][L + 1] offset of each block's values
+    const int32_t* type_count;  // [S] atoms of each type in the system
+    const double* center;       // [N] central-atom contribution
+    const double* k0;           // [N] 4 pi / V times the k = 0 term
+    double center_factor;       // 1 - center_atom_weight
+    int add_k0;
+    // gradients: rows are 3 task + x
+    const int32_t* tasks;       // [n_tasks][4] (i, j, t, row)
+    const int64_t* off_positions;
+    double* out;
+    // the product's tiling
+    int64_t rows;               // rows of one type (values), or 3 tasks
+    int tiles, tiles_even;      // column tiles, and those of the even l
+    int splits, split_k;        // k-vectors [s split_k, (s + 1) split_k) in split s
+    double* partial;            // [splits][types][rows][ld] when splits > 1
+};
+
+// one finished value into its block
+template <bool GRAD>
+__device__ __forceinline__ void lode_store(const LodeArgs& a, int64_t r, int type, int column, double sum) {
+    const bool odd = column >= a.cols.odd0;
+    const int pos = odd ? column - a.cols.odd0 : column;
+    const int lm = pos / a.N, n = pos - lm * a.N;
+    int l = odd ? 1 : 0;
+    while (lode_lm_before(l + 2) <= lm) l += 2;
+    const int mi = lm - lode_lm_before(l), M = 2 * l + 1;
+    const double x = lode_phase(l) * sum;
+    if (GRAD) {
+        const int64_t task = r / 3;
+        const int c = (int)(r - 3 * task);
+        const int32_t* w = a.tasks + 4 * task;
+        const int64_t off = a.off_positions[((size_t)a.species[w[0]] * a.S + w[2]) * (a.L + 1) + l];
+        a.out[off + (((int64_t)w[3] * 3 + c) * M + mi) * a.N + n] = x;
+        return;
+    }
+    const int t = a.present[type], ti = a.species[r];
+    double v = 0.0;
+    if (l == 0) {
+        // central atom (:378-426), then the k = 0 term once per atom of type
+        // t (:635-661)
+        if (t == ti) v -= a.center_factor * a.center[n];
+        if (a.add_k0)
+            for (int j = 0; j < a.type_count[t]; j++) v += a.k0[n];
+    }
+    const int64_t off = a.off_values[((size_t)ti * a.S + t) * (a.L + 1) + l];
+    a.out[off + ((int64_t)a.row[r * a.S + t] * M + mi) * a.N + n] = v + x;
+}
+
+__device__ __forceinline__ void lode_dmma(double (&d)[2], double a, double b) {
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+        : "+d"(d[0]), "+d"(d[1])
+        : "d"(a), "d"(b));
+}
+
+__device__ __forceinline__ void lode_cp16(void* dst, const void* src, bool valid) {
+    const unsigned s = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(s), "l"(src), "r"(valid ? 16 : 0) : "memory");
+}
+
+// Values (spherical_expansion.rs:616-723) and positions gradients (:725-873)
+// as products with T.  A CTA of four warps owns 64 rows x 8 NB columns of one
+// parity of l; a warp computes 16 rows of it.  Per LODE_KB k-vectors the 64
+// rows of the left operand are built from cos and sin (loaded one step ahead
+// into registers) and stored to shared memory, T's rows arrive by cp.async in
+// two buffers.  Bound by the FP64 tensor pipe (2 x rows x k x columns flops;
+// about 36 TFLOP/s); 64 rows keep the reads of T and of cos / sin, both from
+// L2, below it, and 128 registers (four CTAs per SM) hide the two barriers of
+// a step.  Values of 1000 atoms, 3 types, 4522 k-vectors and 392 coefficients
+// (10.6 GFLOP): 0.51 ms = 20.7 TFLOP/s; 0.68 ms with three CTAs per SM and
+// three splits; 2.33 ms as a sum over k on the CUDA cores, eight centres and
+// four coefficients a thread.
+template <int NB, bool GRAD>
+__global__ void __launch_bounds__(LODE_THREADS, GRAD ? 3 : 4) lode_gemm_kernel(LodeArgs a) {
+    constexpr int BN = 8 * NB;
+    constexpr int LDB = ((BN + 11) / 16) * 16 + 4;  // >= BN, 4 (mod 16) doubles
+    __shared__ __align__(16) double As[LODE_ROWS * LODE_LDA];
+    __shared__ __align__(16) double Bs[2][LODE_KB * LDB];
+    __shared__ __align__(16) double Ks[2][3][LODE_KB];  // values: Ct, St; gradients: gdf, k-vectors apart
+    const int64_t row_tile = blockIdx.x / a.tiles;
+    const int tile = (int)(blockIdx.x - row_tile * a.tiles);
+    const int type = blockIdx.y, split = blockIdx.z;
+    const bool odd = tile >= a.tiles_even;
+    const int col0 = odd ? a.cols.odd0 + (tile - a.tiles_even) * BN : tile * BN;
+    const int n_cols = min(BN, (odd ? a.cols.odd0 + a.cols.n_odd : a.cols.n_even) - col0);
+    const int64_t row0 = row_tile * LODE_ROWS;
+    const int kb = split * a.split_k, ke = min(a.Kp, kb + a.split_k);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+    // this thread's part of the left operand: one row, eight k-vectors
+    const int ar = threadIdx.x >> 1, ak = (threadIdx.x & 1) * 8;
+    const int64_t r = row0 + ar;
+    const bool row_ok = r < a.rows;
+    int i = 0, j = 0, t = 0, x = 0;
+    bool same_type = false;
+    if (GRAD) {
+        const int64_t task = row_ok ? r / 3 : 0;
+        x = row_ok ? (int)(r - 3 * task) : 0;
+        i = a.tasks[4 * task];
+        j = a.tasks[4 * task + 1];
+        t = a.tasks[4 * task + 2];
+        same_type = a.species[i] == t;
+    } else {
+        i = row_ok ? (int)r : 0;
+        t = a.present[type];
+    }
+    const double* ci = a.C + (size_t)i * a.Kp + ak;
+    const double* si = a.Sn + (size_t)i * a.Kp + ak;
+    const double* cj = a.C + (size_t)j * a.Kp + ak;
+    const double* sj = a.Sn + (size_t)j * a.Kp + ak;
+    double c8[8], s8[8];
+    auto load8 = [&](const double* src, double(&v)[8]) {
 #pragma unroll
-    for (int q = 0; q < LODE_Q; q++) acc[q][0] = acc[q][1] = acc[q][2] = 0.0;
-    for (int k0 = 0; k0 < a.K; k0 += LODE_CHUNK) {
-        const int nk = min(LODE_CHUNK, a.K - k0);
-        __syncthreads();
-        for (int kk = threadIdx.x; kk < nk; kk += blockDim.x) {
-            const int k = k0 + kk;
-            const double ci = a.C[(size_t)i * a.K + k], si = a.Sn[(size_t)i * a.K + k];
-            const double cj = a.C[(size_t)j * a.K + k], sj = a.Sn[(size_t)j * a.K + k];
-            // real / imaginary part of i e^{i k (r_i - r_j)}
-            double even = 2.0 * (si * cj - ci * sj);
-            double odd = -2.0 * (ci * cj + si * sj);
-            if (i == j) {
-                // -sum_{j != i}: from the structure factor per centre
-                const double ct = a.Ct[(size_t)t * a.K + k], st = a.St[(size_t)t * a.K + k];
-                const double real = 2.0 * (ci * ct + si * st);
-                const double imag = 2.0 * (si * ct - ci * st);
-                if (t == ti) {
-                    even = -(1.0 * imag - even);
-                    odd = -(-1.0 * real - odd);
-                } else {
-                    even = -1.0 * imag;
-                    odd = -(-1.0) * real;
+        for (int q = 0; q < 4; q++) {
+            const double2 w = __ldg(reinterpret_cast<const double2*>(src) + q);
+            v[2 * q] = w.x;
+            v[2 * q + 1] = w.y;
+        }
+    };
+    auto issue = [&](int k, int buf) {
+        for (int q = threadIdx.x; q < LODE_KB * (BN / 2); q += LODE_THREADS) {
+            const int kk = q / (BN / 2), c = 2 * (q - kk * (BN / 2));
+            // columns past the parity's end: zeros, nothing read
+            const bool ok = c < n_cols;
+            lode_cp16(&Bs[buf][kk * LDB + c], a.T + (size_t)(k + kk) * a.cols.ld + (ok ? col0 + c : 0), ok);
+        }
+        if (!GRAD && threadIdx.x < LODE_KB) {
+            const int half = threadIdx.x / (LODE_KB / 2), q = 2 * (threadIdx.x % (LODE_KB / 2));
+            lode_cp16(&Ks[buf][half][q], (half ? a.St : a.Ct) + (size_t)t * a.Kp + k + q, true);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    double acc[2][NB][2];
+#pragma unroll
+    for (int m = 0; m < 2; m++)
+#pragma unroll
+        for (int n = 0; n < NB; n++) acc[m][n][0] = acc[m][n][1] = 0.0;
+
+    if (kb < ke) {
+        issue(kb, 0);
+        load8(ci + kb, c8);
+        load8(si + kb, s8);
+    }
+    int buf = 0;
+    for (int k = kb; k < ke; k += LODE_KB, buf ^= 1) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();  // T's rows are there, and the last step's operands are done with
+        double w[8];
+        if (GRAD) {
+            double cj8[8], sj8[8];
+            load8(cj + k, cj8);
+            load8(sj + k, sj8);
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                const int kk = k + ak + q;
+                // real / imaginary part of i e^{i k (r_i - r_j)}
+                const double pair = a.gdf[kk] * (odd ? -2.0 * (c8[q] * cj8[q] + s8[q] * sj8[q])
+                                                     : 2.0 * (s8[q] * cj8[q] - c8[q] * sj8[q]));
+                double f = pair;
+                if (i == j) {
+                    // -sum_{j != i}: from the structure factor per centre
+                    const double ct = a.Ct[(size_t)t * a.Kp + kk], st = a.St[(size_t)t * a.Kp + kk];
+                    const double sum = odd ? 2.0 * (c8[q] * ct + s8[q] * st) : -2.0 * (s8[q] * ct - c8[q] * st);
+                    f = same_type ? sum + pair : sum;
                 }
+                w[q] = row_ok ? f * a.kvec[3 * kk + x] : 0.0;
             }
-            pe[kk] = even * a.gdf[k];
-            po[kk] = odd * a.gdf[k];
-            kn[kk] = a.knorm[k];
-            kd[kk][0] = a.kdir[3 * k];
-            kd[kk][1] = a.kdir[3 * k + 1];
-            kd[kk][2] = a.kdir[3 * k + 2];
+        } else {
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                // structure factor per centre (:143-155), real or imaginary part
+                const double ct = Ks[buf][0][ak + q], st = Ks[buf][1][ak + q];
+                w[q] = row_ok ? 2.0 * (odd ? s8[q] * ct - c8[q] * st : c8[q] * ct + s8[q] * st) : 0.0;
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            *reinterpret_cast<double2*>(&As[ar * LODE_LDA + ak + 2 * q]) = make_double2(w[2 * q], w[2 * q + 1]);
+        if (k + LODE_KB < ke) {
+            issue(k + LODE_KB, buf ^ 1);
+            load8(ci + k + LODE_KB, c8);
+            load8(si + k + LODE_KB, s8);
         }
         __syncthreads();
+        const double* A0 = As + (16 * warp + (lane >> 2)) * LODE_LDA + (lane & 3);
+        const double* B0 = Bs[buf] + (lane & 3) * LDB + (lane >> 2);
 #pragma unroll
-        for (int q = 0; q < LODE_Q; q++) {
-            const int o = o0 + q * LODE_THREADS + threadIdx.x;
-            if (o >= outs) continue;
-            const bool oddl = l_of(o / a.N) & 1;
-            const double* p = oddl ? po : pe;
-            const double* Tk = a.T + (size_t)k0 * outs + o;
-            int kk = 0;
-            for (; kk + 4 <= nk; kk += 4) {
-                double tv[4];
+        for (int st = 0; st < LODE_KB / 4; st++) {
+            const double a0 = A0[4 * st], a1 = A0[8 * LODE_LDA + 4 * st];
 #pragma unroll
-                for (int u = 0; u < 4; u++) tv[u] = Tk[(size_t)(kk + u) * outs];
-#pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    const double s = p[kk + u] * tv[u] * kn[kk + u];
-                    acc[q][0] += s * kd[kk + u][0];
-                    acc[q][1] += s * kd[kk + u][1];
-                    acc[q][2] += s * kd[kk + u][2];
-                }
-            }
-            for (; kk < nk; kk++) {
-                const double s = p[kk] * Tk[(size_t)kk * outs] * kn[kk];
-                acc[q][0] += s * kd[kk][0];
-                acc[q][1] += s * kd[kk][1];
-                acc[q][2] += s * kd[kk][2];
+            for (int n = 0; n < NB; n++) {
+                const double b = B0[4 * st * LDB + 8 * n];
+                lode_dmma(acc[0][n], a0, b);
+                lode_dmma(acc[1][n], a1, b);
             }
         }
     }
 #pragma unroll
-    for (int q = 0; q < LODE_Q; q++) {
-        const int o = o0 + q * LODE_THREADS + threadIdx.x;
-        if (o >= outs) continue;
-        const int lm = o / a.N, n = o - lm * a.N, l = l_of(lm), mi = lm - l * l;
-        const double phase = lode_phase(l);
-        const int64_t off = a.off_positions[((size_t)ti * a.S + t) * (a.L + 1) + l];
-        for (int x = 0; x < 3; x++)
-            a.out[off + (((int64_t)r * 3 + x) * (2 * l + 1) + mi) * a.N + n] = phase * acc[q][x];
+    for (int m = 0; m < 2; m++) {
+        const int64_t ro = row0 + 16 * warp + 8 * m + (lane >> 2);
+        if (ro >= a.rows) continue;
+#pragma unroll
+        for (int n = 0; n < NB; n++)
+#pragma unroll
+            for (int e = 0; e < 2; e++) {
+                const int c = 8 * n + 2 * (lane & 3) + e;
+                if (c >= n_cols) continue;
+                if (a.splits > 1)
+                    a.partial[(((int64_t)split * gridDim.y + type) * a.rows + ro) * a.cols.ld + col0 + c] = acc[m][n][e];
+                else
+                    lode_store<GRAD>(a, ro, type, col0 + c, acc[m][n][e]);
+            }
+    }
+}
+
+// the splits' sums added in order, thread per (row, column)
+template <bool GRAD>
+__global__ void __launch_bounds__(256) lode_splits_kernel(LodeArgs a, int n_types) {
+    const int64_t item = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t per_split = (int64_t)n_types * a.rows * a.cols.ld;
+    if (item >= per_split) return;
+    const int64_t tr = item / a.cols.ld;
+    const int column = (int)(item - tr * a.cols.ld);
+    if (column >= a.cols.n_even && column < a.cols.odd0) return;
+    if (column >= a.cols.odd0 + a.cols.n_odd) return;
+    double sum = 0.0;
+    for (int s = 0; s < a.splits; s++) sum += a.partial[s * per_split + item];
+    const int type = (int)(tr / a.rows);
+    lode_store<GRAD>(a, tr - type * a.rows, type, column, sum);
+}
+
+// Tiles and splits of one product.  The column tile is the one of 56 or 64
+// that pads the two parities least (56 divides the 224 + 168 columns of lmax
+// 6, nmax 8 exactly; 64 would do 14 % more).  The k-vectors are split, at
+// least 128 to a split, so that the CTAs fill whole waves of the chip: 1000
+// atoms have 336 CTAs for 592 places, and three splits of them, which fill
+// two thirds of the third wave, took 0.56 ms where the rule's choice takes
+// 0.51.  A split costs two steps (its prologue and its share of the sums).
+template <bool GRAD>
+void launch_lode_gemm(LodeArgs a, int64_t rows, int n_types, DeviceArena& arena, cudaStream_t stream) {
+    if (rows == 0 || n_types == 0) return;
+    auto tiles = [&](int bn, int n) { return (n + bn - 1) / bn; };
+    const int t7 = tiles(56, a.cols.n_even) + tiles(56, a.cols.n_odd), t8 = tiles(64, a.cols.n_even) + tiles(64, a.cols.n_odd);
+    const int nb = t7 * 7 < t8 * 8 ? 7 : 8;
+    a.rows = rows;
+    a.tiles_even = tiles(8 * nb, a.cols.n_even);
+    a.tiles = a.tiles_even + tiles(8 * nb, a.cols.n_odd);
+    const int64_t row_tiles = (rows + LODE_ROWS - 1) / LODE_ROWS;
+    const int64_t ctas = row_tiles * a.tiles * n_types;
+    const int steps = a.Kp / LODE_KB, resident = 148 * (GRAD ? 3 : 4);
+    int best = 1;
+    double best_time = 1e300;
+    for (int q = 1; q <= std::max(1, std::min(32, steps / 8)); q++) {
+        const int64_t waves = (ctas * q + resident - 1) / resident;
+        const double time = (double)waves * ((steps + q - 1) / q + 2);
+        if (time < 0.98 * best_time) {
+            best_time = time;
+            best = q;
+        }
+    }
+    a.split_k = (steps + best - 1) / best * LODE_KB;
+    a.splits = (a.Kp + a.split_k - 1) / a.split_k;
+    if (row_tiles * a.tiles > 0x7fffffffLL) throw invalid_parameter("the LODE product is too large for one launch");
+    if (a.splits > 1) a.partial = arena.alloc<double>("lode.partial", (int64_t)a.splits * n_types * rows * a.cols.ld);
+    const dim3 grid((unsigned)(row_tiles * a.tiles), (unsigned)n_types, (unsigned)a.splits);
+    if (nb == 7) lode_gemm_kernel<7, GRAD><<<grid, LODE_THREADS, 0, stream>>>(a);
+    else lode_gemm_kernel<8, GRAD><<<grid, LODE_THREADS, 0, stream>>>(a);
+    CUDA_CHECK(cudaGetLastError());
+    if (a.splits > 1) {
+        const int64_t items = (int64_t)n_types * rows * a.cols.ld;
+        lode_splits_kernel<GRAD><<<(unsigned)((items + 255) / 256), 256, 0, stream>>>(a, n_types);
+        CUDA_CHECK(cudaGetLastError());
     }
 }
 
@@ -609,28 +753,49 @@ LodeEngine::~LodeEngine() {
     for (void* p : table_buffers_) cudaFree(p);
 }
 
+namespace {
+
+// arrays of different types one after the other, for one copy to the device
+struct HostPack {
+    std::vector<unsigned char> bytes;
+    template <typename T>
+    size_t add(const std::vector<T>& v) {
+        const size_t at = bytes.size();
+        bytes.resize(at + (std::max<size_t>(1, v.size() * sizeof(T)) + 255) / 256 * 256);
+        if (!v.empty()) std::memcpy(bytes.data() + at, v.data(), v.size() * sizeof(T));
+        return at;
+    }
+};
+
+}  // namespace
+
 void LodeEngine::upload_tables() {
     int dev = 0;
     CUDA_CHECK(cudaGetDevice(&dev));
     if (tables_ready_ && dev == device_) return;
     if (tables_ready_) throw invalid_parameter("a calculator can only be used on the device it first ran on");
     device_ = dev;
-    auto putv = [&](const std::vector<double>& v) {
-        void* d = nullptr;
-        CUDA_CHECK(cudaMalloc(&d, std::max<size_t>(8, v.size() * sizeof(double))));
-        if (!v.empty()) CUDA_CHECK(cudaMemcpy(d, v.data(), v.size() * sizeof(double), cudaMemcpyHostToDevice));
-        table_buffers_.push_back(d);
-        return (const double*)d;
-    };
-    d_ylm_.lmax = ylm_.lmax;
-    d_ylm_.A = putv(ylm_.A);
-    d_ylm_.B = putv(ylm_.B);
-    d_ylm_.sq_plus = putv(ylm_.sq_plus);
-    d_ylm_.sq_minus = putv(ylm_.sq_minus);
-    d_ylm_.sq_2l1 = putv(ylm_.sq_2l1);
-    d_ylm_.sq_half = putv(ylm_.sq_half);
-    d_ylm_.sq_ll1 = putv(ylm_.sq_ll1);
-    d_ylm_.inv_ll = putv(ylm_.inv_ll);
+    // every table in one allocation and one copy
+    HostPack pack;
+    const size_t at[] = {pack.add(ylm_.A),          pack.add(ylm_.B),          pack.add(ylm_.sq_plus),
+                         pack.add(ylm_.sq_minus),   pack.add(ylm_.sq_2l1),     pack.add(ylm_.sq_half),
+                         pack.add(ylm_.sq_ll1),     pack.add(ylm_.inv_ll),     pack.add(tables_.positions),
+                         pack.add(tables_.values),  pack.add(tables_.derivs),  pack.add(tables_.knot_offset),
+                         pack.add(tables_.knot_count)};
+    unsigned char* d = nullptr;
+    CUDA_CHECK(cudaMalloc(&d, pack.bytes.size()));
+    table_buffers_.push_back(d);
+    CUDA_CHECK(cudaMemcpy(d, pack.bytes.data(), pack.bytes.size(), cudaMemcpyHostToDevice));
+    auto dbl = [&](int k) { return reinterpret_cast<const double*>(d + at[k]); };
+    d_ylm_ = {ylm_.lmax, dbl(0), dbl(1), dbl(2), dbl(3), dbl(4), dbl(5), dbl(6), dbl(7)};
+    d_spline_.lmax = tables_.h.max_angular;
+    d_spline_.nmax = tables_.h.nmax();
+    d_spline_.splined = tables_.positions.empty() ? 0 : 1;
+    d_spline_.positions = dbl(8);
+    d_spline_.values = dbl(9);
+    d_spline_.derivs = dbl(10);
+    d_spline_.knot_offset = reinterpret_cast<const int32_t*>(d + at[11]);
+    d_spline_.knot_count = reinterpret_cast<const int32_t*>(d + at[12]);
     tables_ready_ = true;
 }
 
@@ -761,8 +926,6 @@ std::unique_ptr<TensorMap> LodeEngine::compute(const std::vector<HostSystem>& sy
     CUDA_CHECK(cudaEventRecord(ev0, stream));
 
     int64_t atom_offset = 0;
-    const int64_t* d_offv = put(arena_, "lode.off_values", off_values, stream);
-    const int64_t* d_offp = put(arena_, "lode.off_positions", off_positions, stream);
     for (size_t s = 0; s < systems.size(); s++) {
         const HostSystem& sys = systems[s];
         const int n = (int)sys.n_atoms;
@@ -774,86 +937,94 @@ std::unique_ptr<TensorMap> LodeEngine::compute(const std::vector<HostSystem>& sy
         const double volume = std::fabs(c[0] * (c[4] * c[8] - c[5] * c[7]) - c[1] * (c[3] * c[8] - c[5] * c[6]) +
                                         c[2] * (c[3] * c[7] - c[4] * c[6]));
         const double global = 4.0 * M_PI / volume;
-        std::vector<double> kvec(3 * (size_t)K), gdf(K), radial((size_t)K * (L + 1) * N);
+        const int Kp = (K + LODE_KB - 1) / LODE_KB * LODE_KB;
+        // the radial integral is evaluated on the device from its spline; the
+        // analytic integral comes from here
+        std::vector<double> kvec(3 * (size_t)Kp, 0.0), gdf(Kp, 0.0), radial(h.splined ? 0 : (size_t)K * (L + 1) * N);
 #pragma omp parallel for schedule(static)
         for (int k = 0; k < K; k++) {
             for (int x = 0; x < 3; x++) kvec[3 * k + x] = kv.norm[k] * kv.direction[3 * k + x];
             gdf[k] = global * tables_.density_fourier(kv.norm[k]);
+            if (h.splined) continue;
             for (int l = 0; l <= L; l++) tables_.radial(l, kv.norm[k], &radial[((size_t)k * (L + 1) + l) * N], nullptr);
         }
-        std::vector<double> k0(N), center = tables_.center;
+        std::vector<double> k0(N);
         for (int q = 0; q < N; q++) k0[q] = global * tables_.k0[q];
         std::vector<int32_t> count(S, 0);
         for (int32_t t : sys_species[s]) count[t]++;
 
+        // the atoms by type, and the types of this system
+        std::vector<int32_t> sorted_atoms, type_start(S + 1, 0), present;
+        for (int t = 0; t < S; t++) {
+            type_start[t + 1] = type_start[t] + count[t];
+            if (count[t]) present.push_back(t);
+        }
+        sorted_atoms.resize(n);
+        {
+            std::vector<int32_t> next(type_start.begin(), type_start.end() - 1);
+            for (int i = 0; i < n; i++) sorted_atoms[next[sys_species[s][i]]++] = i;
+        }
+
+        // everything the kernels read from here, in one copy
+        HostPack pack;
+        const size_t o_species = pack.add(sys_species[s]), o_kvec = pack.add(kvec), o_norm = pack.add(kv.norm),
+                     o_dir = pack.add(kv.direction), o_gdf = pack.add(gdf), o_radial = pack.add(radial),
+                     o_sorted = pack.add(sorted_atoms), o_start = pack.add(type_start), o_present = pack.add(present),
+                     o_rows = pack.add(rows[s]), o_count = pack.add(count), o_center = pack.add(tables_.center),
+                     o_k0 = pack.add(k0), o_offv = pack.add(off_values), o_offp = pack.add(off_positions),
+                     o_positions = d_positions ? 0 : pack.add(sys.positions);
+        const unsigned char* d_pack = put(arena_, "lode.pack", pack.bytes, stream);
+        auto doubles = [&](size_t at) { return reinterpret_cast<const double*>(d_pack + at); };
+        auto ints = [&](size_t at) { return reinterpret_cast<const int32_t*>(d_pack + at); };
         LodeArgs a{};
-        a.n_atoms = n;
-        a.K = K;
+        a.Kp = Kp;
         a.S = S;
+        a.cols = lode_columns(L, N);
         a.L = L;
         a.N = N;
-        a.species = put(arena_, "lode.species", sys_species[s], stream);
-        double* d_kvec = put(arena_, "lode.kvec", kvec, stream);
-        a.kvec = d_kvec;
-        a.knorm = put(arena_, "lode.knorm", kv.norm, stream);
-        a.kdir = put(arena_, "lode.kdir", kv.direction, stream);
-        a.gdf = put(arena_, "lode.gdf", gdf, stream);
-        const double* d_radial = put(arena_, "lode.radial", radial, stream);
-        double* T = arena_.alloc<double>("lode.T", (int64_t)K * L2 * N);
-        double* C = arena_.alloc<double>("lode.cos", (int64_t)n * K);
-        double* Sn = arena_.alloc<double>("lode.sin", (int64_t)n * K);
-        double* Ct = arena_.alloc<double>("lode.cos_sum", (int64_t)S * K);
-        double* St = arena_.alloc<double>("lode.sin_sum", (int64_t)S * K);
+        a.species = ints(o_species);
+        a.kvec = doubles(o_kvec);
+        a.gdf = doubles(o_gdf);
+        // cos, sin, their sums by type and T in one allocation
+        const int64_t phases = (int64_t)n * Kp, sums = (int64_t)S * Kp;
+        double* C = arena_.alloc<double>("lode.work", 2 * phases + 2 * sums + (int64_t)Kp * a.cols.ld);
+        double* Sn = C + phases;
+        double* Ct = Sn + phases;
+        double* St = Ct + sums;
+        double* T = St + sums;
         a.T = T;
         a.C = C;
         a.Sn = Sn;
         a.Ct = Ct;
         a.St = St;
-        a.row = put(arena_, "lode.rows", rows[s], stream);
-        a.off_values = d_offv;
-        a.off_positions = d_offp;
-        a.type_count = put(arena_, "lode.type_count", count, stream);
-        a.center = put(arena_, "lode.center", center, stream);
-        a.k0 = put(arena_, "lode.k0", k0, stream);
+        a.present = ints(o_present);
+        a.row = ints(o_rows);
+        a.off_values = reinterpret_cast<const int64_t*>(d_pack + o_offv);
+        a.off_positions = reinterpret_cast<const int64_t*>(d_pack + o_offp);
+        a.type_count = ints(o_count);
+        a.center = doubles(o_center);
+        a.k0 = doubles(o_k0);
         a.center_factor = 1.0 - h.center_atom_weight;
         a.add_k0 = (h.exponent == 0 || h.exponent > 3) ? 1 : 0;
         a.out = d_out;
-
-        const double* positions = nullptr;
-        if (d_positions) {
-            positions = d_positions + 3 * atom_offset;
-        } else {
-            positions = put(arena_, "lode.positions", sys.positions, stream);
-        }
-        lode_projection_kernel<<<(K + 127) / 128, 128, 0, stream>>>(K, L, N, a.kdir, d_radial, d_ylm_, T);
+        const double* positions = d_positions ? d_positions + 3 * atom_offset : doubles(o_positions);
+        // k-vectors per CTA of the projection: at most 8 and 48 KB of shared memory
+        const size_t per_k = sizeof(double) * (size_t)((L + 1) * (L + 2) / 2 + L2 + (L + 1) * N);
+        const int kc = (int)std::max<size_t>(1, std::min<size_t>(8, 48 * 1024 / per_k));
+        lode_projection_kernel<<<(Kp + kc - 1) / kc, 128, kc * per_k, stream>>>(
+            K, Kp, kc, N, a.cols, doubles(o_dir), doubles(o_norm), h.splined ? nullptr : doubles(o_radial), d_spline_, d_ylm_,
+            T);
         CUDA_CHECK(cudaGetLastError());
-        const int64_t nk = (int64_t)n * K;
-        lode_phases_kernel<<<(unsigned)((nk + 255) / 256), 256, 0, stream>>>(n, K, positions, d_kvec, C, Sn);
+        const int64_t nk = (int64_t)n * Kp;
+        lode_phases_kernel<<<(unsigned)((nk + 255) / 256), 256, 0, stream>>>(n, K, Kp, positions, a.kvec, C, Sn);
         CUDA_CHECK(cudaGetLastError());
-        lode_type_sums_kernel<<<(S * K + 255) / 256, 256, 0, stream>>>(n, K, S, a.species, C, Sn, Ct, St);
+        lode_type_sums_kernel<<<dim3((Kp + 31) / 32, S), 256, 0, stream>>>(K, Kp, ints(o_sorted), ints(o_start), a.gdf, C,
+                                                                          Sn, Ct, St);
         CUDA_CHECK(cudaGetLastError());
-        // groups of LODE_GROUP centres of one species
-        std::vector<int32_t> groups;
-        for (int t = 0; t < S; t++) {
-            std::vector<int32_t> members;
-            for (int i = 0; i < n; i++)
-                if (sys_species[s][i] == t) members.push_back(i);
-            for (size_t q = 0; q < members.size(); q += LODE_GROUP)
-                for (int c2 = 0; c2 < LODE_GROUP; c2++)
-                    groups.push_back(q + c2 < members.size() ? members[q + c2] : -1);
-        }
-        const int n_groups = (int)(groups.size() / LODE_GROUP);
-        const int32_t* d_groups = put(arena_, "lode.groups", groups, stream);
-        const unsigned tiles = (unsigned)((L2 * N + LODE_THREADS * LODE_Q - 1) / (LODE_THREADS * LODE_Q));
-        if (n_groups > 0) {
-            lode_values_kernel<<<dim3((unsigned)(n_groups * S), tiles), LODE_THREADS, 0, stream>>>(a, d_groups, n_groups);
-            CUDA_CHECK(cudaGetLastError());
-        }
+        launch_lode_gemm<false>(a, n, (int)present.size(), arena_, stream);
         if (g.positions && !tasks[s].empty()) {
-            const int n_tasks = (int)(tasks[s].size() / 4);
             a.tasks = put(arena_, "lode.tasks", tasks[s], stream);
-            lode_gradients_kernel<<<dim3((unsigned)n_tasks, tiles), LODE_THREADS, 0, stream>>>(a, n_tasks);
-            CUDA_CHECK(cudaGetLastError());
+            launch_lode_gemm<true>(a, 3 * (int64_t)(tasks[s].size() / 4), 1, arena_, stream);
         }
         // the per-system buffers are reused by the next system
         CUDA_CHECK(cudaStreamSynchronize(stream));

@@ -68,6 +68,7 @@ class LodeEngine {
     LodeTables tables_;
     YlmTables ylm_;
     DeviceYlm d_ylm_{};
+    DeviceRadial d_spline_{};  // the radial integral's spline over |k|
     std::vector<void*> table_buffers_;
     bool tables_ready_ = false;
     int device_ = -1;
