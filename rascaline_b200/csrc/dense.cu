@@ -36,6 +36,7 @@
 #include <cstdlib>
 #include <type_traits>
 
+#include "centre_expansion.cuh"
 #include "dense.hpp"
 #include "pair_math.cuh"
 
@@ -557,7 +558,7 @@ __global__ void __launch_bounds__(128) dense_pair_adjoint_fused(DenseArgs<T> a, 
         g2 += AY * u2 + Bf * gy[2];
     };
     ylm_rows<T, 8, true>(
-        a.tab.ylm, u0, u1, u2,
+        a.tab.ylm_const, u0, u1, u2,
         [&](int l) {
             spline_row<T, NCAP>(a.tab.spline, l, r, R, dR);
 #pragma unroll
@@ -834,17 +835,39 @@ void launch_dense_forward(const DenseArgs<T>& a, int64_t n_pairs, cudaStream_t s
         if (a.marks) CUDA_CHECK(cudaEventRecord(a.marks[k], stream));
     };
     mark(0);
-    if (a.gradient_features) launch_features<T, true>(a, n_pairs, stream);
-    else launch_features<T, false>(a, n_pairs, stream);
+    CentreArgs<T> ca{};
+    ca.n_centres = a.n_atoms;
+    ca.n_species = a.n_species;
+    ca.centre_species = a.atom_species;
+    ca.seg_offset = a.seg_offset;
+    ca.dir_code = a.dir_code;
+    ca.distance = a.pairs.distance;
+    ca.vector = a.pairs.vector;
+    ca.spline = a.tab.spline;
+    ca.ylm = a.tab.ylm_const;
+    ca.cut = a.cut;
+    ca.self_contribution = a.tab.self_contribution;
+    ca.coef = a.coef;
+    // the surrogate, the analytic integral, lmax > 8 and nmax > 16 take the
+    // pair records
+    const bool by_centre = !a.gradient_features && a.surrogate == nullptr && centre_expansion_supported(a.tab);
+    if (!by_centre) {
+        if (a.gradient_features) launch_features<T, true>(a, n_pairs, stream);
+        else launch_features<T, false>(a, n_pairs, stream);
+    }
     mark(1);
     if (a.n_atoms == 0) {
         mark(2);
         mark(3);
         return;
     }
-    dense_expansion<T><<<(unsigned)(a.n_atoms * a.n_species),
-                         coefficient_threads(a.layout.L2 * ((a.nmax + 1) / 2)), 0, stream>>>(a);
-    CUDA_CHECK(cudaGetLastError());
+    if (by_centre) {
+        launch_centre_expansion(ca, stream);
+    } else {
+        dense_expansion<T><<<(unsigned)(a.n_atoms * a.n_species),
+                             coefficient_threads(a.layout.L2 * ((a.nmax + 1) / 2)), 0, stream>>>(a);
+        CUDA_CHECK(cudaGetLastError());
+    }
     mark(2);
     if (a.values == nullptr) {  // the expansion alone
         mark(3);

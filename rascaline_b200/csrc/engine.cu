@@ -20,6 +20,7 @@
 #include "dense.hpp"
 #include "engine.hpp"
 #include "plan.hpp"
+#include "soap_math.cuh"
 
 namespace fb200 {
 
@@ -353,12 +354,19 @@ void Engine::upload_tables() {
     CUDA_CHECK(cudaDeviceGetDefaultMemPool(&pool, dev));
     uint64_t threshold = UINT64_MAX;
     CUDA_CHECK(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &threshold));
+    // every table in one allocation, filled by one copy at the end
+    const size_t room = ((size_t)1 << 18) + sizeof(double) * (radial_.positions.size() * 4 + radial_.values.size() * 16 +
+                                                             radial_.ortho.size() * 4);
+    unsigned char* base = nullptr;
+    CUDA_CHECK(cudaMalloc(&base, room));
+    table_buffers_.push_back(base);
+    std::vector<unsigned char> staged;
     auto put = [&](const void* src, size_t bytes) -> void* {
-        void* d = nullptr;
-        CUDA_CHECK(cudaMalloc(&d, bytes > 0 ? bytes : 8));
-        if (bytes) CUDA_CHECK(cudaMemcpy(d, src, bytes, cudaMemcpyHostToDevice));
-        table_buffers_.push_back(d);
-        return d;
+        const size_t at = staged.size();
+        staged.resize(at + (std::max<size_t>(bytes, 8) + 255) / 256 * 256);
+        if (staged.size() > room) throw internal_error("the calculator's tables outgrow their allocation");
+        if (bytes) std::memcpy(staged.data() + at, src, bytes);
+        return base + at;
     };
     auto putv = [&](const std::vector<double>& v) { return (const double*)put(v.data(), v.size() * sizeof(double)); };
     d_radial_.lmax = radial_.lmax;
@@ -393,11 +401,96 @@ void Engine::upload_tables() {
     dense_d_.spline = {d_radial_.lmax, d_radial_.nmax, d_radial_.splined, d_radial_.knot_offset,
                        d_radial_.knot_count, d_radial_.positions, d_radial_.values, d_radial_.derivs};
     dense_d_.self_contribution = d_self_;
+    // channels with the same knots
+    auto& spline = dense_d_.spline;
+    std::vector<double> quads;
+    if (radial_.splined && radial_.lmax < spline.MAX_CHANNELS) {
+        const int N = radial_.nmax;
+        auto begin = [&](int l) { return radial_.positions.begin() + radial_.knot_offset[l]; };
+        std::vector<std::vector<int>> channels;  // of every level
+        for (int l = 0; l <= radial_.lmax; l++) {
+            size_t v = 0;
+            while (v < channels.size() && !(radial_.knot_count[channels[v][0]] == radial_.knot_count[l] &&
+                                            std::equal(begin(l), begin(l) + radial_.knot_count[l], begin(channels[v][0]))))
+                v++;
+            if (v == channels.size()) channels.emplace_back();
+            channels[v].push_back(l);
+        }
+        if ((int)channels.size() <= spline.MAX_LEVELS) {
+            // bins finer than most intervals: the search after the lookup is
+            // a step or two
+            constexpr int BINS = 2048;
+            const double scale = BINS / h_.cutoff;
+            std::vector<int32_t> lut;
+            std::vector<double> grid;
+            for (size_t v = 0; v < channels.size(); v++) {
+                const int count = radial_.knot_count[channels[v][0]];
+                const double* pos = &*begin(channels[v][0]);
+                for (int b = 0; b < BINS; b++) lut.push_back(soap::spline_interval(pos, count, b / scale));
+                spline.first_knot[v] = (int)(grid.size() / 2);
+                spline.level_knots[v] = count;
+                spline.quad_pitch[v] = (int)channels[v].size() * N;
+                const size_t start = quads.size() / 4;
+                quads.resize(quads.size() + (size_t)count * spline.quad_pitch[v] * 4, 0.0);
+                for (size_t i = 0; i < channels[v].size(); i++) {
+                    spline.level_of[channels[v][i]] = (int)v;
+                    spline.first_quad[channels[v][i]] = (int)(start + i * N);
+                }
+                for (int k = 0; k < count; k++) {
+                    grid.push_back(pos[k]);
+                    grid.push_back(k + 1 < count ? 1.0 / (pos[k + 1] - pos[k]) : 0.0);
+                    if (k + 1 == count) break;
+                    for (int l : channels[v])
+                        for (int n = 0; n < N; n++) {
+                            const size_t from = ((size_t)radial_.knot_offset[l] + k) * N + n;
+                            double* to = &quads[4 * ((size_t)spline.first_quad[l] + (size_t)k * spline.quad_pitch[v] + n)];
+                            to[0] = radial_.values[from];
+                            to[1] = radial_.derivs[from];
+                            to[2] = radial_.values[from + N];
+                            to[3] = radial_.derivs[from + N];
+                        }
+                }
+            }
+            spline.levels = (int)channels.size();
+            spline.lut_bins = BINS;
+            spline.lut_scale = scale;
+            spline.lut = (const int32_t*)put(lut.data(), lut.size() * sizeof(int32_t));
+            spline.knots = (const double2*)putv(grid);
+            spline.quads = putv(quads);
+        }
+    }
     dense_f_.ylm = {ylm_.lmax,          putf(ylm_.A),      putf(ylm_.B),       putf(ylm_.sq_plus), putf(ylm_.sq_minus),
                     putf(ylm_.sq_2l1), putf(ylm_.sq_half), putf(ylm_.sq_ll1), putf(ylm_.inv_ll)};
     dense_f_.spline = {d_radial_.lmax,        d_radial_.nmax,       d_radial_.splined,    d_radial_.knot_offset,
                        d_radial_.knot_count,  d_radial_.positions, putf(radial_.values), putf(radial_.derivs)};
+    dense_f_.spline.levels = spline.levels;
+    dense_f_.spline.lut_bins = spline.lut_bins;
+    dense_f_.spline.lut_scale = spline.lut_scale;
+    std::copy(std::begin(spline.level_of), std::end(spline.level_of), dense_f_.spline.level_of);
+    std::copy(std::begin(spline.first_quad), std::end(spline.first_quad), dense_f_.spline.first_quad);
+    std::copy(std::begin(spline.quad_pitch), std::end(spline.quad_pitch), dense_f_.spline.quad_pitch);
+    std::copy(std::begin(spline.level_knots), std::end(spline.level_knots), dense_f_.spline.level_knots);
+    std::copy(std::begin(spline.first_knot), std::end(spline.first_knot), dense_f_.spline.first_knot);
+    dense_f_.spline.knots = spline.knots;
+    dense_f_.spline.lut = spline.lut;
+    if (spline.levels > 0) dense_f_.spline.quads = putf(quads);
+    if (ylm_.lmax <= YlmConst<double>::LCAP) {
+        auto fill = [&](auto& c) {
+            c.lmax = ylm_.lmax;
+            std::copy(ylm_.A.begin(), ylm_.A.end(), c.A);
+            std::copy(ylm_.B.begin(), ylm_.B.end(), c.B);
+            std::copy(ylm_.sq_plus.begin(), ylm_.sq_plus.end(), c.sq_plus);
+            std::copy(ylm_.sq_minus.begin(), ylm_.sq_minus.end(), c.sq_minus);
+            std::copy(ylm_.sq_2l1.begin(), ylm_.sq_2l1.end(), c.sq_2l1);
+            std::copy(ylm_.sq_half.begin(), ylm_.sq_half.end(), c.sq_half);
+            std::copy(ylm_.sq_ll1.begin(), ylm_.sq_ll1.end(), c.sq_ll1);
+            std::copy(ylm_.inv_ll.begin(), ylm_.inv_ll.end(), c.inv_ll);
+        };
+        fill(dense_d_.ylm_const);
+        fill(dense_f_.ylm_const);
+    }
     dense_f_.self_contribution = putf(radial_.self_contribution);
+    CUDA_CHECK(cudaMemcpy(base, staged.data(), staged.size(), cudaMemcpyHostToDevice));
     tables_ready_ = true;
 }
 
@@ -518,7 +611,7 @@ std::unique_ptr<TensorMap> Engine::compute(int kind, std::vector<HostSystem>& sy
     FeatureLayout layout = FeatureLayout::make(h_.max_angular, h_.nmax(), g.any());
     // the spherical expansion builds its pair terms itself (fused kernel) or
     // reads them from per-pair records
-    const bool fused_se = !by_pair && n_atoms > 0 && se_fused_enabled() && se_fused_supported(layout, d_radial_);
+    const bool fused_se = !by_pair && n_atoms > 0 && se_fused_enabled() && se_fused_supported(layout, d_radial_, dense_d_);
     double* features = fused_se ? nullptr : arena_.alloc<double>("features", pairs.count * layout.stride);
     int32_t* status = arena_.alloc<int32_t>("status", 1);
     CUDA_CHECK(cudaMemsetAsync(status, 0, sizeof(int32_t), stream));
@@ -598,7 +691,7 @@ std::unique_ptr<TensorMap> Engine::compute(int kind, std::vector<HostSystem>& sy
         se.strain = g.strain ? arena_.alloc<double>("se.strain", n_atoms * S * 9 * K) : nullptr;
         se.cellg = g.cell ? arena_.alloc<double>("se.cell", n_atoms * S * 9 * K) : nullptr;
         CUDA_CHECK(cudaEventRecord(ev[7], stream));
-        if (fused_se) launch_se_fused(se, pairs, d_radial_, d_ylm_, cut, stream);
+        if (fused_se) launch_se_fused(se, pairs, d_radial_, d_ylm_, cut, dense_d_, stream);
         else launch_se_accumulate(se, stream);
         CUDA_CHECK(cudaEventRecord(ev[3], stream));
     }
@@ -1042,7 +1135,10 @@ std::unique_ptr<DenseState> Engine::forward_dense(int precision, std::vector<Hos
     const bool keep = backward_follows && precision == 32 && active_surrogate_ != nullptr && !expansion;
     const FeatureLayout layout = FeatureLayout::make(h_.max_angular, h_.nmax(), keep);
     const size_t feature_bytes = T_size * (size_t)std::max<int64_t>(P, 1) * layout.stride;
-    void* features = keep ? st->alloc(feature_bytes) : arena_.alloc_bytes("dense.features", feature_bytes);
+    // the expansion by centre needs no pair records
+    const bool records = keep || (precision == 32 ? active_surrogate_ != nullptr || !centre_expansion_supported(dense_f_)
+                                                  : !centre_expansion_supported(dense_d_));
+    void* features = keep ? st->alloc(feature_bytes) : records ? arena_.alloc_bytes("dense.features", feature_bytes) : nullptr;
     if (keep) st->features_grad = features;
     cudaEvent_t* marks = dense_marks();
     if (precision == 64) {

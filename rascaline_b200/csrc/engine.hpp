@@ -106,6 +106,15 @@ struct DeviceYlmT {
 };
 using DeviceYlm = DeviceYlmT<double>;
 
+// the same for lmax <= 8 by value: as a kernel argument they are operands from
+// constant memory where the loops over (l, m) are unrolled
+template <typename T>
+struct YlmConst {
+    static constexpr int LCAP = 8, N = (LCAP + 1) * (LCAP + 2) / 2;
+    int lmax = -1;
+    T A[N], B[N], sq_plus[N], sq_minus[N], sq_2l1[LCAP + 1], sq_half[LCAP + 1], sq_ll1[LCAP + 1], inv_ll[LCAP + 1];
+};
+
 // spline tables with values / derivatives in T (knot positions in FP64)
 template <typename T>
 struct DeviceSplineT {
@@ -115,15 +124,41 @@ struct DeviceSplineT {
     const double* positions;
     const T* values;
     const T* derivs;
+    // Channels with the same knots share a level (levels = 0 when there are
+    // more than MAX_LEVELS): per level the knots (position, 1 / distance to the
+    // next), the interval at the start of every bin of width 1 / lut_scale, and
+    // per (knot, channel of the level, n) the value and derivative at the knot
+    // and at the next one
+    static constexpr int MAX_LEVELS = 3, MAX_CHANNELS = 9;
+    int levels = 0, lut_bins = 0;
+    double lut_scale = 0.0;
+    int level_of[MAX_CHANNELS] = {};      // [lmax + 1]
+    int first_quad[MAX_CHANNELS] = {};    // [lmax + 1] of (knot 0, n = 0)
+    int quad_pitch[MAX_LEVELS] = {};      // quads per knot
+    int level_knots[MAX_LEVELS] = {};     // number of knots
+    int first_knot[MAX_LEVELS] = {};
+    const double2* knots = nullptr;
+    const int32_t* lut = nullptr;         // [levels][lut_bins]
+    const T* quads = nullptr;             // [...][4]
 };
 
 // device tables of the dense kernels in one arithmetic type
 template <typename T>
 struct DenseTables {
     DeviceYlmT<T> ylm;
+    YlmConst<T> ylm_const;  // for lmax <= 8
     DeviceSplineT<T> spline;
     const T* self_contribution = nullptr;
 };
+
+// whether the expansion by centre (centre_expansion.cuh) takes these tables;
+// the analytic integral, channels with more than MAX_LEVELS kinds of knots,
+// lmax > 8 and nmax > 16 take the kernels over pair records
+constexpr int CE_NMAX = 16;
+template <typename T>
+bool centre_expansion_supported(const DenseTables<T>& t) {
+    return t.spline.splined && t.spline.levels > 0 && t.ylm_const.lmax >= 0 && t.spline.nmax <= CE_NMAX;
+}
 
 struct CutoffParams {
     double rc, width;
@@ -176,10 +211,10 @@ void launch_pair_features(const DevicePairs& pairs, const DeviceRadial& radial, 
 void launch_se_accumulate(const SeArgs& args, cudaStream_t stream);
 // pair_features + se_accumulate in one kernel (the pair terms built in shared
 // memory, args.features unused), for lmax <= 8 and splined radial
-// integrals; bit-identical results
-bool se_fused_supported(const FeatureLayout& layout, const DeviceRadial& radial);
+// integrals; bit-identical results.  Without gradients, one CTA per centre.
+bool se_fused_supported(const FeatureLayout& layout, const DeviceRadial& radial, const DenseTables<double>& tables);
 void launch_se_fused(const SeArgs& args, const DevicePairs& pairs, const DeviceRadial& radial, const DeviceYlm& ylm,
-                     const CutoffParams& cut, cudaStream_t stream);
+                     const CutoffParams& cut, const DenseTables<double>& tables, cudaStream_t stream);
 // whether the drop-in's spherical expansion uses the fused kernel (default)
 // or the two-kernel path; FEATOMIC_B200_FUSED_SE=0 selects the two kernels
 bool se_fused_enabled();

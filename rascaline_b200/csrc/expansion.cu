@@ -24,6 +24,7 @@
 #include <algorithm>
 #include <cstdlib>
 
+#include "centre_expansion.cuh"
 #include "engine.hpp"
 #include "pair_math.cuh"
 #include "soap_math.cuh"
@@ -541,15 +542,34 @@ bool se_fused_enabled() {
 
 void set_se_fused_enabled(bool enabled) { fused_state = enabled ? 1 : 0; }
 
-bool se_fused_supported(const FeatureLayout& layout, const DeviceRadial& radial) {
+bool se_fused_supported(const FeatureLayout& layout, const DeviceRadial& radial, const DenseTables<double>& tables) {
+    if (!layout.with_grad && centre_expansion_supported(tables)) return true;
     const size_t bytes = sizeof(double) * fused_shared_doubles(layout.lmax, layout.nmax, layout.with_grad);
     const int items = layout.L2 * ((layout.nmax + 1) / 2);
     return radial.splined && layout.lmax <= LMAX_SMALL && items <= 256 && bytes <= 160 * 1024;
 }
 
 void launch_se_fused(const SeArgs& args, const DevicePairs& pairs, const DeviceRadial& radial, const DeviceYlm& ylm,
-                     const CutoffParams& cut, cudaStream_t stream) {
+                     const CutoffParams& cut, const DenseTables<double>& tables, cudaStream_t stream) {
     if (args.n_centres == 0) return;
+    if (!args.layout.with_grad && centre_expansion_supported(tables)) {
+        // values alone: bit-identical to the kernels here
+        CentreArgs<double> ca{};
+        ca.n_centres = args.n_centres;
+        ca.n_species = args.n_species;
+        ca.centre_species = args.centre_species;
+        ca.seg_offset = args.seg_offset;
+        ca.dir_code = args.dir_code;
+        ca.distance = pairs.distance;
+        ca.vector = pairs.vector;
+        ca.spline = tables.spline;
+        ca.ylm = tables.ylm_const;
+        ca.cut = cut;
+        ca.self_contribution = args.self_contribution;
+        ca.coef = args.coef;
+        launch_centre_expansion(ca, stream);
+        return;
+    }
     const FeatureLayout& L = args.layout;
     const int items = L.L2 * ((L.nmax + 1) / 2);
     const int threads = std::max(32, (items + 31) / 32 * 32);

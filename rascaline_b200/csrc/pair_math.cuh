@@ -119,6 +119,28 @@ __device__ void ylm_compute(const DeviceYlmT<T>& tab, T ux, T uy, T uz, T* __res
     }
 }
 
+// The angles of a unit direction, as ylm_compute derives them
+template <typename T>
+struct YlmAngles {
+    T ct, st, cp, sp;
+};
+
+template <typename T>
+__device__ __forceinline__ YlmAngles<T> ylm_angles(T ux, T uy, T uz) {
+    YlmAngles<T> a;
+    const T sxy = hypot(ux, uy);
+    a.ct = uz;
+    a.st = sxy;
+    if (sxy > T(soap::DBL_EPS)) {
+        a.cp = ux / sxy;
+        a.sp = uy / sxy;
+    } else {
+        a.cp = T(1);
+        a.sp = T(0);
+    }
+    return a;
+}
+
 // The same harmonics row by row: begin(l) is called before row l and
 // visit(l, m, y+, y-, g+, g-) for m = 0..l with Y_l^{+m}, Y_l^{-m} (y- unused
 // for m = 0) and their gradients w.r.t. the unit direction (g+/g- all zero
@@ -126,24 +148,16 @@ __device__ void ylm_compute(const DeviceYlmT<T>& tab, T ux, T uy, T uz, T* __res
 // the results are identical, but in l-outer order: three rows of Legendre
 // polynomials live in registers instead of a local-memory table.  For
 // LCAP <= 8 (the register arrays are unrolled).
-template <typename T, int LCAP, bool GRAD, typename Begin, typename Visit>
-__device__ __forceinline__ void ylm_rows(const DeviceYlmT<T>& tab, T ux, T uy, T uz, Begin begin, Visit visit) {
+template <typename T, int LCAP, bool GRAD, typename Tables, typename Begin, typename Visit>
+__device__ __forceinline__ void ylm_rows(const Tables& tab, T ux, T uy, T uz, Begin begin, Visit visit) {
     static_assert(LCAP <= 8, "ylm_rows keeps (LCAP + 1) x 4 Legendre values in registers");
     const int lmax = tab.lmax;
     const T SQRT_1_OVER_2PI = T(0.3989422804014327);
     const T SQRT_3 = T(1.7320508075688772);
     const T SQRT_3_OVER_2 = T(1.224744871391589);
     const T SQRT_2 = T(1.4142135623730951);
-    const T sxy = hypot(ux, uy);
-    const T ct = uz, st = sxy;
-    T cp, sp;
-    if (sxy > T(soap::DBL_EPS)) {
-        cp = ux / sxy;
-        sp = uy / sxy;
-    } else {
-        cp = T(1);
-        sp = T(0);
-    }
+    const YlmAngles<T> angles = ylm_angles(ux, uy, uz);
+    const T ct = angles.ct, st = angles.st, cp = angles.cp, sp = angles.sp;
     // cos(m phi), sin(m phi) by the recursion of :300-306
     T cm[LCAP + 1], sm[LCAP + 1];
     {
@@ -232,28 +246,7 @@ __device__ __forceinline__ void ylm_rows(const DeviceYlmT<T>& tab, T ux, T uy, T
 }
 
 // The same harmonics split by column m, for one thread per (direction, m).
-// The direction's angles, as ylm_compute derives them:
-template <typename T>
-struct YlmAngles {
-    T ct, st, cp, sp;
-};
-
-template <typename T>
-__device__ __forceinline__ YlmAngles<T> ylm_angles(T ux, T uy, T uz) {
-    YlmAngles<T> a;
-    const T sxy = hypot(ux, uy);
-    a.ct = uz;
-    a.st = sxy;
-    if (sxy > T(soap::DBL_EPS)) {
-        a.cp = ux / sxy;
-        a.sp = uy / sxy;
-    } else {
-        a.cp = T(1);
-        a.sp = T(0);
-    }
-    return a;
-}
-
+//
 // Column m of the associated Legendre table, P(l, m) for l = m..lmax, written
 // to P[lidx(l, m)].  The recursions of ylm_compute restricted to one column
 // (every P(l, m) depends on P(l - 1, m), P(l - 2, m) and the diagonal chain
