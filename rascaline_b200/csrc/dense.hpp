@@ -45,7 +45,7 @@ struct DenseArgs {
     T* grad_coef;         // [n_atoms][S][K]
     T* pair_grad;         // [n_pairs][3] dL/dr_ij
     T* grad_positions;    // [n_atoms][3]
-    T* atom_partial;      // [n_atoms][18] strain then cell sums over the atom's own pairs
+    T* atom_partial;      // [18][n_atoms] strain then cell sums over the atom's own pairs
     T* grad_strain;       // [n_systems][9] or null
     T* grad_cell;         // [n_systems][9] or null
     int32_t* status;
