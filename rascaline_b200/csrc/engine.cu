@@ -1094,7 +1094,7 @@ std::unique_ptr<DenseState> Engine::forward_dense(int precision, std::vector<Hos
     CUDA_CHECK(cudaMemcpyAsync(st->atom_species, atom_species.data(), sizeof(int32_t) * n_atoms,
                                cudaMemcpyHostToDevice, stream));
 
-    // neighbour list (kernel a), then a private copy for the backward pass
+    // neighbour list (kernel a)
     std::vector<NlSystem> nls;
     int64_t atom_off = 0, cell_off = 0;
     for (auto& s : systems) {
@@ -1103,24 +1103,15 @@ std::unique_ptr<DenseState> Engine::forward_dense(int precision, std::vector<Hos
         atom_off += s.n_atoms;
         nls.push_back(n);
     }
-    const int64_t P = nl_.build(nls, atom_system, d_positions, n_atoms, arena_, stream);
+    // the list is written into the state's own memory: the backward pass and
+    // the calculator's next list don't share it
+    const int64_t P = nl_.build(nls, atom_system, d_positions, n_atoms, arena_, stream,
+                                [&](size_t bytes) { return st->alloc(bytes); });
     st->n_pairs = P;
-    st->pairs.count = P;
-    st->pairs.first = (int32_t*)st->alloc(sizeof(int32_t) * P);
-    st->pairs.second = (int32_t*)st->alloc(sizeof(int32_t) * P);
-    st->pairs.distance = (double*)st->alloc(sizeof(double) * P);
-    st->pairs.vector = (double*)st->alloc(sizeof(double) * 3 * P);
-    st->pairs.shift = (int32_t*)st->alloc(sizeof(int32_t) * 3 * P);
-    st->pair_start = (int64_t*)st->alloc(sizeof(int64_t) * (n_atoms + 1));
-    if (P > 0) {
-        CUDA_CHECK(cudaMemcpyAsync(st->pairs.first, nl_.pairs.first, 4 * P, cudaMemcpyDeviceToDevice, stream));
-        CUDA_CHECK(cudaMemcpyAsync(st->pairs.second, nl_.pairs.second, 4 * P, cudaMemcpyDeviceToDevice, stream));
-        CUDA_CHECK(cudaMemcpyAsync(st->pairs.distance, nl_.pairs.distance, 8 * P, cudaMemcpyDeviceToDevice, stream));
-        CUDA_CHECK(cudaMemcpyAsync(st->pairs.vector, nl_.pairs.vector, 24 * P, cudaMemcpyDeviceToDevice, stream));
-        CUDA_CHECK(cudaMemcpyAsync(st->pairs.shift, nl_.pairs.shift, 12 * P, cudaMemcpyDeviceToDevice, stream));
-    }
-    CUDA_CHECK(cudaMemcpyAsync(st->pair_start, nl_.pair_start, sizeof(int64_t) * (n_atoms + 1),
-                               cudaMemcpyDeviceToDevice, stream));
+    st->pairs = nl_.pairs;
+    st->pair_start = const_cast<int64_t*>(nl_.pair_start);
+    nl_.pairs = DevicePairs();
+    nl_.pair_start = nullptr;
 
     // direction segments, coefficients, power spectrum
     st->dir_code = (int32_t*)st->alloc(sizeof(int32_t) * 2 * P);

@@ -5,6 +5,7 @@
 
 #include <cstdint>
 #include <map>
+#include <functional>
 #include <memory>
 #include <string>
 #include <vector>
@@ -78,8 +79,11 @@ class NeighborBuilder {
     DevicePairs pairs;
     // [n_atoms + 1] first pair of every atom (pairs are sorted by first atom)
     const int64_t* pair_start = nullptr;
+    // the pairs and pair_start come from `allocate` when it is given (they
+    // outlive the builder's next list), from the arena otherwise
     int64_t build(const std::vector<NlSystem>& systems, const std::vector<int32_t>& atom_system,
-                  const double* d_positions, int64_t n_atoms, DeviceArena& arena, cudaStream_t stream);
+                  const double* d_positions, int64_t n_atoms, DeviceArena& arena, cudaStream_t stream,
+                  const std::function<void*(size_t)>& allocate = nullptr);
 };
 
 // ---------------------------------------------------------------------------

@@ -91,61 +91,116 @@ __global__ void nl_fill_cells(const int32_t* __restrict__ cell_of, int64_t n_ato
     cell_atoms[cell_start[c] + slot] = (int32_t)g;
 }
 
-// Candidate pairs of atom g, enumerated by one warp: the lanes stride over
-// the atoms of every neighbouring cell.  `visit(keep, j, shift, v, d2)` is
+// Candidate pairs of atom g, enumerated by one warp: the atoms of every
+// neighbouring cell, cell after cell.  `visit(keep, j, shift, v, d2)` is
 // called by every lane for every round (keep is false for lanes without a
 // kept pair), so that the caller can use warp-wide ballots.
+//
+// Latency bound.  The lanes look up 32 cells at a time and then stride over
+// the atoms of all of them, two rounds' loads in flight, so that a round is 32
+// candidates whatever the cells hold (8 to 15 atoms a cell left half of the
+// lanes idle and made 27 rounds, each behind its own cell lookup, of what are
+// 7 to 13).  Count and write together: 64 atoms 40 -> 14 us, 1000 atoms 84 ->
+// 46, 20 000 atoms 358 -> 200; four rounds in flight take too many registers
+// (20 000 atoms 218, 134 128 atoms of molecules 408 against 325).
+constexpr int NL_ROUNDS = 2;
+
 template <typename Visit>
 __device__ __forceinline__ void nl_warp_enumerate(const NlSystem& s, int64_t g, const double* __restrict__ positions,
                                                   const int32_t* __restrict__ cell_of, const int32_t* __restrict__ atom_shift,
                                                   const int32_t* __restrict__ cell_start, const int32_t* __restrict__ cell_count,
                                                   const int32_t* __restrict__ cell_atoms, int lane, Visit visit) {
+    constexpr unsigned ALL = 0xffffffffu;
     const int local = (int)(cell_of[g] - s.cell_offset);
-    const int cz = local % s.n_cells[2];
-    const int cy = (local / s.n_cells[2]) % s.n_cells[1];
-    const int cx = local / (s.n_cells[2] * s.n_cells[1]);
+    const int n0 = s.n_cells[0], n1 = s.n_cells[1], n2 = s.n_cells[2];
+    const int cz = local % n2;
+    const int cy = (local / n2) % n1;
+    const int cx = local / (n2 * n1);
     const int si[3] = {atom_shift[3 * g], atom_shift[3 * g + 1], atom_shift[3 * g + 2]};
     const double pi[3] = {positions[3 * g], positions[3 * g + 1], positions[3 * g + 2]};
-    for (int dx = -s.n_search[0]; dx <= s.n_search[0]; dx++)
-    for (int dy = -s.n_search[1]; dy <= s.n_search[1]; dy++)
-    for (int dz = -s.n_search[2]; dz <= s.n_search[2]; dz++) {
-        int cs[3], ni[3];
-        divmod_i(cx + dx, s.n_cells[0], &cs[0], &ni[0]);
-        divmod_i(cy + dy, s.n_cells[1], &cs[1], &ni[1]);
-        divmod_i(cz + dz, s.n_cells[2], &cs[2], &ni[2]);
-        const int32_t nc = (int32_t)(s.cell_offset + ((int64_t)ni[0] * s.n_cells[1] + ni[1]) * s.n_cells[2] + ni[2]);
-        const int32_t start = cell_start[nc], count = cell_count[nc];
-        for (int32_t q0 = 0; q0 < count; q0 += 32) {
-            const int32_t q = q0 + lane;
-            bool keep = false;
-            int32_t j = -1;
-            int sh[3] = {0, 0, 0};
-            double v[3] = {0.0, 0.0, 0.0};
-            double d2 = 0.0;
-            if (q < count) {
-                j = cell_atoms[start + q];
-                keep = g <= j;
-                for (int k = 0; k < 3; k++) sh[k] = cs[k] + si[k] - atom_shift[3 * (int64_t)j + k];
-                const bool zero = sh[0] == 0 && sh[1] == 0 && sh[2] == 0;
-                if (keep && g == j) {
-                    // self images: one of each +/- shift pair (neighbors.rs:253-286)
-                    const int sum = sh[0] + sh[1] + sh[2];
-                    if (zero || sum < 0 || (sum == 0 && (sh[2] < 0 || (sh[2] == 0 && sh[1] < 0)))) keep = false;
+    const bool infinite = s.infinite;
+    const double cutoff2 = s.cutoff2;
+    const int w1 = 2 * s.n_search[1] + 1, w2 = 2 * s.n_search[2] + 1;
+    const int n_neighbours = (2 * s.n_search[0] + 1) * w1 * w2;
+    for (int c0 = 0; c0 < n_neighbours; c0 += 32) {
+        // this lane's cell
+        const int c = c0 + lane;
+        int cs[3] = {0, 0, 0}, start = 0, count = 0;
+        if (c < n_neighbours) {
+            const int dx = c / (w1 * w2), rest = c - dx * w1 * w2, dy = rest / w2, dz = rest - dy * w2;
+            int ni[3];
+            divmod_i(cx + dx - s.n_search[0], n0, &cs[0], &ni[0]);
+            divmod_i(cy + dy - s.n_search[1], n1, &cs[1], &ni[1]);
+            divmod_i(cz + dz - s.n_search[2], n2, &cs[2], &ni[2]);
+            const int32_t nc = (int32_t)(s.cell_offset + ((int64_t)ni[0] * n1 + ni[1]) * n2 + ni[2]);
+            start = cell_start[nc];
+            count = cell_count[nc];
+        }
+        int last = count;  // candidates of the cells up to this lane's
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const int below = __shfl_up_sync(ALL, last, off);
+            if (lane >= off) last += below;
+        }
+        const int total = __shfl_sync(ALL, last, 31);
+        const int first = last - count;
+        for (int q0 = 0; q0 < total; q0 += 32 * NL_ROUNDS) {
+            // NL_ROUNDS rounds of 32 candidates, their loads in flight together
+            int32_t j[NL_ROUNDS];
+            int sh[NL_ROUNDS][3];
+            double pj[NL_ROUNDS][3];
+            bool keep[NL_ROUNDS];
+#pragma unroll
+            for (int u = 0; u < NL_ROUNDS; u++) {
+                const int q = q0 + 32 * u + lane;
+                // the cell of candidate q: the first lane with last > q
+                int owner = 0;
+#pragma unroll
+                for (int step = 16; step > 0; step >>= 1) {
+                    const int probe = __shfl_sync(ALL, last, owner + step - 1);
+                    if (probe <= q) owner += step;
                 }
-                if (s.infinite && !zero) keep = false;
-                if (keep) {
-                    for (int k = 0; k < 3; k++) {
-                        // CellShift::cartesian, neighbors.rs:52-57
-                        const double c = __dadd_rn(__dadd_rn(__dmul_rn(s.H[0 * 3 + k], (double)sh[0]),
-                                                             __dmul_rn(s.H[1 * 3 + k], (double)sh[1])),
-                                                   __dmul_rn(s.H[2 * 3 + k], (double)sh[2]));
-                        v[k] = __dadd_rn(__dsub_rn(positions[3 * (int64_t)j + k], pi[k]), c);
-                    }
-                    d2 = __dadd_rn(__dadd_rn(__dmul_rn(v[0], v[0]), __dmul_rn(v[1], v[1])), __dmul_rn(v[2], v[2]));
-                    keep = d2 < s.cutoff2;
+                const int at = __shfl_sync(ALL, start, owner) + q - __shfl_sync(ALL, first, owner);
+#pragma unroll
+                for (int k = 0; k < 3; k++) sh[u][k] = __shfl_sync(ALL, cs[k], owner);
+                j[u] = q < total ? cell_atoms[at] : -1;
+            }
+#pragma unroll
+            for (int u = 0; u < NL_ROUNDS; u++) {
+                keep[u] = g <= j[u];
+#pragma unroll
+                for (int k = 0; k < 3; k++) {
+                    if (keep[u]) sh[u][k] += si[k] - atom_shift[3 * (int64_t)j[u] + k];
+                    pj[u][k] = keep[u] ? positions[3 * (int64_t)j[u] + k] : 0.0;
                 }
             }
-            visit(keep, j, sh, v, d2);
+#pragma unroll
+            for (int u = 0; u < NL_ROUNDS; u++) {
+                if (q0 + 32 * u >= total) break;
+                double v[3] = {0.0, 0.0, 0.0};
+                double d2 = 0.0;
+                if (keep[u]) {
+                    const bool zero = sh[u][0] == 0 && sh[u][1] == 0 && sh[u][2] == 0;
+                    if (g == j[u]) {
+                        // self images: one of each +/- shift pair (neighbors.rs:253-286)
+                        const int sum = sh[u][0] + sh[u][1] + sh[u][2];
+                        if (zero || sum < 0 || (sum == 0 && (sh[u][2] < 0 || (sh[u][2] == 0 && sh[u][1] < 0)))) keep[u] = false;
+                    }
+                    if (infinite && !zero) keep[u] = false;
+                    if (keep[u]) {
+                        for (int k = 0; k < 3; k++) {
+                            // CellShift::cartesian, neighbors.rs:52-57
+                            const double x = __dadd_rn(__dadd_rn(__dmul_rn(s.H[0 * 3 + k], (double)sh[u][0]),
+                                                                 __dmul_rn(s.H[1 * 3 + k], (double)sh[u][1])),
+                                                       __dmul_rn(s.H[2 * 3 + k], (double)sh[u][2]));
+                            v[k] = __dadd_rn(__dsub_rn(pj[u][k], pi[k]), x);
+                        }
+                        d2 = __dadd_rn(__dadd_rn(__dmul_rn(v[0], v[0]), __dmul_rn(v[1], v[1])), __dmul_rn(v[2], v[2]));
+                        keep[u] = d2 < cutoff2;
+                    }
+                }
+                visit(keep[u], j[u], sh[u], v, d2);
+            }
         }
     }
 }
@@ -174,48 +229,82 @@ __device__ __forceinline__ bool pair_key_less(int32_t j1, const int32_t* s1, int
     return false;
 }
 
-// kept pairs of atom g in enumeration order into `scratch`, then every lane
-// places its pairs at their rank in (second, shift) order
-__global__ void nl_write(const NlSystem* __restrict__ systems, const int32_t* __restrict__ atom_system,
-                         const double* __restrict__ positions, int64_t n_atoms, const int32_t* __restrict__ cell_of,
-                         const int32_t* __restrict__ atom_shift, const int32_t* __restrict__ cell_start,
-                         const int32_t* __restrict__ cell_count, const int32_t* __restrict__ cell_atoms,
-                         const int64_t* __restrict__ pair_start, DevicePairs scratch, DevicePairs pairs) {
-    const int64_t g = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
+constexpr int NL_WARPS = 4;
+constexpr int NL_STAGED = 96;  // kept pairs of an atom that fit in shared memory
+
+// Kept pairs of atom g in enumeration order into shared memory (atoms with
+// more than NL_STAGED of them: into `scratch`), then every lane places its
+// pairs at their rank in (second, shift) order.  With the pairs in shared
+// memory the ranks cost 26 broadcast reads per pair where they were global
+// loads.
+__global__ void __launch_bounds__(32 * NL_WARPS)
+nl_write(const NlSystem* __restrict__ systems, const int32_t* __restrict__ atom_system,
+         const double* __restrict__ positions, int64_t n_atoms, const int32_t* __restrict__ cell_of,
+         const int32_t* __restrict__ atom_shift, const int32_t* __restrict__ cell_start,
+         const int32_t* __restrict__ cell_count, const int32_t* __restrict__ cell_atoms,
+         const int64_t* __restrict__ pair_start, DevicePairs scratch, DevicePairs pairs) {
+    __shared__ int4 keys[NL_WARPS][NL_STAGED];
+    __shared__ double4 data[NL_WARPS][NL_STAGED];  // vector, distance
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t g = (int64_t)blockIdx.x * NL_WARPS + warp;
     if (g >= n_atoms) return;
     const NlSystem& s = systems[atom_system[g]];
     const int64_t base = pair_start[g];
-    int64_t written = 0;
+    const int n = (int)(pair_start[g + 1] - base);
+    const bool staged = n <= NL_STAGED;
+    int written = 0;
     nl_warp_enumerate(s, g, positions, cell_of, atom_shift, cell_start, cell_count, cell_atoms, lane,
                       [&](bool keep, int32_t j, const int* sh, const double* v, double d2) {
                           const unsigned mask = __ballot_sync(0xffffffffu, keep);
                           if (keep) {
-                              const int64_t w = base + written + __popc(mask & ((1u << lane) - 1u));
-                              scratch.second[w] = j;
-                              scratch.distance[w] = __dsqrt_rn(d2);
-                              for (int k = 0; k < 3; k++) {
-                                  scratch.vector[3 * w + k] = v[k];
-                                  scratch.shift[3 * w + k] = sh[k];
+                              const int at = written + __popc(mask & ((1u << lane) - 1u));
+                              const double r = __dsqrt_rn(d2);
+                              if (staged) {
+                                  keys[warp][at] = make_int4(j, sh[0], sh[1], sh[2]);
+                                  data[warp][at] = make_double4(v[0], v[1], v[2], r);
+                              } else {
+                                  const int64_t w = base + at;
+                                  scratch.second[w] = j;
+                                  scratch.distance[w] = r;
+                                  for (int k = 0; k < 3; k++) {
+                                      scratch.vector[3 * w + k] = v[k];
+                                      scratch.shift[3 * w + k] = sh[k];
+                                  }
                               }
                           }
                           written += __popc(mask);
                       });
     __syncwarp();
-    for (int64_t a = lane; a < written; a += 32) {
-        const int32_t j = scratch.second[base + a];
-        const int32_t* sh = &scratch.shift[3 * (base + a)];
-        int64_t rank = 0;
-        for (int64_t b = 0; b < written; b++)
-            if (pair_key_less(scratch.second[base + b], &scratch.shift[3 * (base + b)], j, sh)) rank++;
+    for (int x = lane; x < written; x += 32) {
+        int4 key;
+        double4 d;
+        int rank = 0;
+        if (staged) {
+            key = keys[warp][x];
+            d = data[warp][x];
+            for (int b = 0; b < written; b++) {
+                const int4 o = keys[warp][b];
+                const bool less = o.x != key.x ? o.x < key.x : o.y != key.y ? o.y < key.y : o.z != key.z ? o.z < key.z : o.w < key.w;
+                rank += less ? 1 : 0;
+            }
+        } else {
+            const int32_t* sh = &scratch.shift[3 * (base + x)];
+            key = make_int4(scratch.second[base + x], sh[0], sh[1], sh[2]);
+            const double* v = &scratch.vector[3 * (base + x)];
+            d = make_double4(v[0], v[1], v[2], scratch.distance[base + x]);
+            for (int b = 0; b < written; b++)
+                if (pair_key_less(scratch.second[base + b], &scratch.shift[3 * (base + b)], key.x, sh)) rank++;
+        }
         const int64_t w = base + rank;
         pairs.first[w] = (int32_t)g;
-        pairs.second[w] = j;
-        pairs.distance[w] = scratch.distance[base + a];
-        for (int k = 0; k < 3; k++) {
-            pairs.vector[3 * w + k] = scratch.vector[3 * (base + a) + k];
-            pairs.shift[3 * w + k] = sh[k];
-        }
+        pairs.second[w] = key.x;
+        pairs.distance[w] = d.w;
+        pairs.vector[3 * w] = d.x;
+        pairs.vector[3 * w + 1] = d.y;
+        pairs.vector[3 * w + 2] = d.z;
+        pairs.shift[3 * w] = key.y;
+        pairs.shift[3 * w + 1] = key.z;
+        pairs.shift[3 * w + 2] = key.w;
     }
 }
 
@@ -226,7 +315,8 @@ __global__ void nl_write(const NlSystem* __restrict__ systems, const int32_t* __
 NlSystem make_nl_system(const double* cell, double cutoff, int64_t atom_offset, int64_t n_atoms, int64_t cell_offset);
 
 int64_t NeighborBuilder::build(const std::vector<NlSystem>& systems, const std::vector<int32_t>& atom_system,
-                               const double* d_positions, int64_t n_atoms, DeviceArena& arena, cudaStream_t stream) {
+                               const double* d_positions, int64_t n_atoms, DeviceArena& arena, cudaStream_t stream,
+                               const std::function<void*(size_t)>& allocate) {
     int64_t n_systems = (int64_t)systems.size();
     int64_t n_cells = 0;
     for (auto& s : systems) n_cells = std::max<int64_t>(n_cells, s.cell_offset + (int64_t)s.n_cells[0] * s.n_cells[1] * s.n_cells[2]);
@@ -241,7 +331,8 @@ int64_t NeighborBuilder::build(const std::vector<NlSystem>& systems, const std::
     int32_t* d_cell_fill = arena.alloc<int32_t>("nl.cell_fill", n_cells + 1);
     int32_t* d_cell_atoms = arena.alloc<int32_t>("nl.cell_atoms", n_atoms);
     int64_t* d_pair_count = arena.alloc<int64_t>("nl.pair_count", n_atoms + 1);
-    int64_t* d_pair_start = arena.alloc<int64_t>("nl.pair_start", n_atoms + 1);
+    int64_t* d_pair_start = allocate ? (int64_t*)allocate(sizeof(int64_t) * (n_atoms + 1))
+                                     : arena.alloc<int64_t>("nl.pair_start", n_atoms + 1);
 
     CUDA_CHECK(cudaMemcpyAsync(d_sys, systems.data(), sizeof(NlSystem) * n_systems, cudaMemcpyHostToDevice, stream));
     CUDA_CHECK(cudaMemcpyAsync(d_atom_system, atom_system.data(), sizeof(int32_t) * n_atoms, cudaMemcpyHostToDevice, stream));
@@ -272,11 +363,19 @@ int64_t NeighborBuilder::build(const std::vector<NlSystem>& systems, const std::
     CUDA_CHECK(cudaStreamSynchronize(stream));
     if (total >= (int64_t)INT32_MAX) throw internal_error("too many pairs for the neighbour list");
 
-    pairs.first = arena.alloc<int32_t>("pairs.first", total);
-    pairs.second = arena.alloc<int32_t>("pairs.second", total);
-    pairs.distance = arena.alloc<double>("pairs.distance", total);
-    pairs.vector = arena.alloc<double>("pairs.vector", 3 * total);
-    pairs.shift = arena.alloc<int32_t>("pairs.shift", 3 * total);
+    if (allocate) {
+        pairs.first = (int32_t*)allocate(sizeof(int32_t) * total);
+        pairs.second = (int32_t*)allocate(sizeof(int32_t) * total);
+        pairs.distance = (double*)allocate(sizeof(double) * total);
+        pairs.vector = (double*)allocate(sizeof(double) * 3 * total);
+        pairs.shift = (int32_t*)allocate(sizeof(int32_t) * 3 * total);
+    } else {
+        pairs.first = arena.alloc<int32_t>("pairs.first", total);
+        pairs.second = arena.alloc<int32_t>("pairs.second", total);
+        pairs.distance = arena.alloc<double>("pairs.distance", total);
+        pairs.vector = arena.alloc<double>("pairs.vector", 3 * total);
+        pairs.shift = arena.alloc<int32_t>("pairs.shift", 3 * total);
+    }
     pairs.count = total;
     DevicePairs scratch;
     scratch.second = arena.alloc<int32_t>("nl.scratch.second", total);
@@ -285,7 +384,7 @@ int64_t NeighborBuilder::build(const std::vector<NlSystem>& systems, const std::
     scratch.shift = arena.alloc<int32_t>("nl.scratch.shift", 3 * total);
     scratch.count = total;
     if (n_atoms > 0 && total > 0) {
-        nl_write<<<warp_blocks, threads, 0, stream>>>(d_sys, d_atom_system, d_positions, n_atoms, d_cell_of,
+        nl_write<<<(unsigned)((n_atoms + NL_WARPS - 1) / NL_WARPS), 32 * NL_WARPS, 0, stream>>>(d_sys, d_atom_system, d_positions, n_atoms, d_cell_of,
                                                       d_atom_shift, d_cell_start, d_cell_count, d_cell_atoms,
                                                       d_pair_start, scratch, pairs);
         CUDA_CHECK(cudaGetLastError());
