@@ -357,8 +357,10 @@ void Engine::upload_tables() {
     // every table in one allocation, filled by one copy at the end
     const size_t room = ((size_t)1 << 18) + sizeof(double) * (radial_.positions.size() * 4 + radial_.values.size() * 16 +
                                                              radial_.ortho.size() * 4);
+    // (from the pool: cudaMalloc maps new memory for a block of this size, 2 ms
+    // of the first call of every calculator; the copy below waits for both)
     unsigned char* base = nullptr;
-    CUDA_CHECK(cudaMalloc(&base, room));
+    CUDA_CHECK(cudaMallocAsync((void**)&base, room, cudaStreamLegacy));
     table_buffers_.push_back(base);
     std::vector<unsigned char> staged;
     auto put = [&](const void* src, size_t bytes) -> void* {
@@ -594,9 +596,12 @@ std::unique_ptr<TensorMap> Engine::compute(int kind, std::vector<HostSystem>& sy
 
     // ---- pair indices to the host, then the per-pair features run on the GPU
     // while the host builds the metadata ----------------------------------------
-    // the power spectrum builds its neighbourhood tables on the device: the
-    // host needs no pair list
-    const bool device_tables = ps && n_atoms > 0;
+    // the power spectrum and the spherical expansion build their neighbourhood
+    // tables on the device: the host needs no pair list.  (The expansion of a
+    // caller's own pairs, in any order, keeps the host's.)
+    const bool device_tables = !by_pair && n_atoms > 0 && (ps || !user_pairs);
+    // the entries (unique neighbours) are the rows of the positions gradients
+    const bool device_entries = device_tables && g.positions;
     std::vector<int32_t> h_first(device_tables ? 0 : pairs.count), h_second(device_tables ? 0 : pairs.count),
         h_shift(by_pair ? 3 * pairs.count : 0);
     if (pairs.count && !device_tables) {
@@ -653,7 +658,7 @@ std::unique_ptr<TensorMap> Engine::compute(int kind, std::vector<HostSystem>& sy
             CUDA_CHECK(cudaEventRecord(ev[14], stream));
             CUDA_CHECK(cudaStreamWaitEvent(up, ev[14], 0));
             // pinned staging: [entry offsets][entries][species counts][species mask]
-            nb_capacity = 2 * pairs.count + n_atoms;
+            nb_capacity = g.positions ? 2 * pairs.count + n_atoms : 0;
             const size_t b_offset = sizeof(int64_t) * (n_atoms + 1), b_entries = sizeof(PsEntry) * nb_capacity;
             const size_t b_count = sizeof(int32_t) * n_atoms * S;
             char* host = (char*)staging(b_offset + b_entries + b_count + n_atoms * S);
@@ -664,18 +669,20 @@ std::unique_ptr<TensorMap> Engine::compute(int kind, std::vector<HostSystem>& sy
             // the species counts come back as soon as they are counted (ev[12]),
             // before the scan and the fill of the entries
             nb = launch_neighborhoods(pairs, d_species, d_dir, d_seg, S, n_atoms, arena_, up, nb_host_count,
-                                      nb_host_mask, ev[12]);
-            // the entries go back to the host (for the labels) on a stream of
-            // their own, so that the contraction kernels, which join the copy
-            // stream, do not wait for this copy
-            cudaStream_t back = readback_stream();
-            CUDA_CHECK(cudaEventRecord(ev[15], up));
-            CUDA_CHECK(cudaStreamWaitEvent(back, ev[15], 0));
-            CUDA_CHECK(cudaMemcpyAsync(nb_host_offset, nb.entry_offset, sizeof(int64_t) * (n_atoms + 1),
-                                       cudaMemcpyDeviceToHost, back));
-            CUDA_CHECK(cudaMemcpyAsync(nb_host_entries, nb.entries, sizeof(PsEntry) * nb_capacity,
-                                       cudaMemcpyDeviceToHost, back));
-            CUDA_CHECK(cudaEventRecord(ev[13], back));
+                                      nb_host_mask, ev[12], device_entries);
+            if (device_entries) {
+                // the entries go back to the host (for the labels) on a stream of
+                // their own, so that the contraction kernels, which join the copy
+                // stream, do not wait for this copy
+                cudaStream_t back = readback_stream();
+                CUDA_CHECK(cudaEventRecord(ev[15], up));
+                CUDA_CHECK(cudaStreamWaitEvent(back, ev[15], 0));
+                CUDA_CHECK(cudaMemcpyAsync(nb_host_offset, nb.entry_offset, sizeof(int64_t) * (n_atoms + 1),
+                                           cudaMemcpyDeviceToHost, back));
+                CUDA_CHECK(cudaMemcpyAsync(nb_host_entries, nb.entries, sizeof(PsEntry) * nb_capacity,
+                                           cudaMemcpyDeviceToHost, back));
+                CUDA_CHECK(cudaEventRecord(ev[13], back));
+            }
         }
         se.centre_species = d_species;
         se.seg_offset = d_seg;
@@ -731,7 +738,7 @@ std::unique_ptr<TensorMap> Engine::compute(int kind, std::vector<HostSystem>& sy
                                 : plan_spherical_expansion(nh, h_, g);
     // the device's entries into the host tables, for the labels
     auto load_entries = [&]() {
-        if (!device_tables) return;
+        if (!device_entries) return;
         CUDA_CHECK(cudaEventSynchronize(ev[13]));
         nh.entry_offset.assign(nb_host_offset, nb_host_offset + n_atoms + 1);
         const int64_t n_entries = nh.entry_offset[n_atoms];
@@ -860,19 +867,19 @@ std::unique_ptr<TensorMap> Engine::compute(int kind, std::vector<HostSystem>& sy
             so.strain = se.strain;
             so.cellg = se.cellg;
             so.dir_code = se.dir_code;
-            so.n_rows = (int64_t)plan.row_centre.size();
-            so.row_centre = upload(arena_, "so.row_centre", plan.row_centre, up);
-            so.row_block = upload(arena_, "so.row_block", plan.row_block, up);
-            so.row_sample = upload(arena_, "so.row_sample", plan.row_sample, up);
-            so.n_grad_rows = (int64_t)plan.grad_block.size();
-            so.grad_block = upload(arena_, "so.grad_block", plan.grad_block, up);
-            so.grad_row = upload(arena_, "so.grad_row", plan.grad_row, up);
-            so.grad_centre = upload(arena_, "so.grad_centre", plan.grad_centre, up);
-            so.grad_atom = upload(arena_, "so.grad_atom", plan.grad_atom, up);
-            so.grad_d0 = upload(arena_, "so.grad_d0", plan.grad_d0, stream);
-            so.grad_d1 = upload(arena_, "so.grad_d1", plan.grad_d1, stream);
-            so.block_l = upload(arena_, "so.block_l", plan.block_l, up);
-            so.block_species = upload(arena_, "so.block_species", plan.block_species, up);
+            so.n_centres = nh.n_atoms;
+            so.slot_offset = upload(arena_, "ps.slot_offset", plan.slot_offset, up);
+            so.slots = upload(arena_, "ps.slots", plan.slots, up);
+            so.slot_row = upload(arena_, "ps.slot_row", plan.slot_row, up);
+            if (g.positions && device_tables) {
+                so.entry_offset = nb.entry_offset;
+                so.entries = nb.entries;
+                so.entry_cum = nb.entry_cum;
+            } else if (g.positions) {
+                so.entry_offset = upload(arena_, "nb.entry_offset", nh.entry_offset, up);
+                so.entries = upload(arena_, "nb.entries", nh.entries, up);
+                so.entry_cum = upload(arena_, "nb.entry_cum", nh.entry_cum, up);
+            }
             so.off_values = upload(arena_, "so.offv", offv, up);
             so.off_positions = upload(arena_, "so.offp", offp, up);
             so.off_strain = upload(arena_, "so.offs", offs, up);
@@ -883,6 +890,11 @@ std::unique_ptr<TensorMap> Engine::compute(int kind, std::vector<HostSystem>& sy
             CUDA_CHECK(cudaEventRecord(ev[9], stream));
             t_launch = std::chrono::steady_clock::now();
             launch_se_output(so, g.positions, g.strain, g.cell, stream);
+            // the labels only describe the output: written while the kernels run
+            auto t_labels = std::chrono::steady_clock::now();
+            load_entries();
+            fill_spherical_expansion_labels(nh, g, plan);
+            meta_extra += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_labels).count();
         }
         CUDA_CHECK(cudaEventRecord(ev[4], stream));
         int32_t h_status = 0;
@@ -893,9 +905,10 @@ std::unique_ptr<TensorMap> Engine::compute(int kind, std::vector<HostSystem>& sy
                                  "`cutoff`, or increasing the Gaussian's `width`.");
         }
     } else {
-        if (ps) {
+        if (!by_pair) {
             load_entries();
-            fill_power_spectrum_labels(nh, g, plan);
+            if (ps) fill_power_spectrum_labels(nh, g, plan);
+            else fill_spherical_expansion_labels(nh, g, plan);
         }
         for (int k : {7, 3, 8, 9, 4}) CUDA_CHECK(cudaEventRecord(ev[k], stream));
     }

@@ -293,11 +293,13 @@ struct DeviceNeighborhoods {
 };
 // When `host_count` / `host_mask` are given, the species counts and masks are
 // copied to them right after the counting kernel and `counted` is recorded
-// there, before the scan and the fill.
+// there, before the scan and the fill.  Without `with_entries` the counts and
+// masks are all there is.
 DeviceNeighborhoods launch_neighborhoods(const DevicePairs& pairs, const int32_t* atom_species, const int32_t* dir_code,
                                          const int64_t* seg_offset, int n_species, int64_t n_atoms, DeviceArena& arena,
                                          cudaStream_t stream, int32_t* host_count = nullptr,
-                                         uint8_t* host_mask = nullptr, cudaEvent_t counted = nullptr);
+                                         uint8_t* host_mask = nullptr, cudaEvent_t counted = nullptr,
+                                         bool with_entries = true);
 
 // Spherical expansion output scatter (spherical_expansion calculator)
 struct SeOutArgs {
@@ -308,21 +310,17 @@ struct SeOutArgs {
     const double* strain;
     const double* cellg;
     const int32_t* dir_code;
-    // one entry per (block, sample)
-    int64_t n_rows;
-    const int32_t* row_centre;   // global centre
-    const int32_t* row_block;    // block index
-    const int32_t* row_sample;   // sample index in the block
-    // one entry per gradient row
-    int64_t n_grad_rows;
-    const int32_t* grad_block;
-    const int64_t* grad_row;     // row index in the block
-    const int32_t* grad_centre;
-    const int32_t* grad_atom;    // neighbour (== centre for self rows)
-    const int32_t* grad_d0;      // direction range
-    const int32_t* grad_d1;
-    const int32_t* block_l;
-    const int32_t* block_species;
+    int64_t n_centres;
+    // the slots of every centre (block of l = 0, sample, neighbour species),
+    // and the first gradient row of each
+    const int64_t* slot_offset;
+    const PsKeySlot* slots;
+    const int64_t* slot_row;
+    // unique neighbours of every centre and their prefix counts (positions
+    // gradients only)
+    const int64_t* entry_offset;
+    const PsEntry* entries;
+    const int32_t* entry_cum;
     const int64_t* off_values;
     const int64_t* off_positions;
     const int64_t* off_strain;

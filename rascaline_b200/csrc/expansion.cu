@@ -431,64 +431,100 @@ __global__ void __launch_bounds__(256, 2) se_fused_kernel(SeArgs a, DevicePairs 
     }
 }
 
+__device__ __forceinline__ int l_of_lm(int lm) {
+    int l = (int)sqrtf((float)lm);
+    while (l * l > lm) l--;
+    while ((l + 1) * (l + 1) <= lm) l++;
+    return l;
+}
+
 // spherical_expansion calculator output: values / strain / cell of one
-// (block, sample) row per CTA
-__global__ void se_output_rows_kernel(SeOutArgs a, int do_strain, int do_cell) {
-    const int64_t row = blockIdx.x;
-    const int K = (a.lmax + 1) * (a.lmax + 1) * a.nmax;
-    const int c = a.row_centre[row];
-    const int blk = a.row_block[row];
-    const int s = a.row_sample[row];
-    const int l = a.block_l[blk];
-    const int t = a.block_species[blk];
-    const int width = (2 * l + 1) * a.nmax;
-    const int64_t src = ((int64_t)c * a.n_species + t);
-    const int start = l * l * a.nmax;
-    for (int q = threadIdx.x; q < width; q += blockDim.x)
-        a.out[a.off_values[blk] + (int64_t)s * width + q] = a.coef[src * K + start + q];
-    if (do_strain) {
-        for (int q = threadIdx.x; q < 9 * width; q += blockDim.x) {
-            int x = q / width, w = q - x * width;
-            a.out[a.off_strain[blk] + (int64_t)s * 9 * width + q] = a.strain[(src * 9 + x) * K + start + w];
-        }
-    }
-    if (do_cell) {
-        for (int q = threadIdx.x; q < 9 * width; q += blockDim.x) {
-            int x = q / width, w = q - x * width;
-            a.out[a.off_cell[blk] + (int64_t)s * 9 * width + q] = a.cellg[(src * 9 + x) * K + start + w];
+// centre's slots per CTA, the blocks of every l
+__global__ void __launch_bounds__(128) se_output_rows_kernel(SeOutArgs a, int do_strain, int do_cell) {
+    const int64_t c = blockIdx.x;
+    const int N = a.nmax, K = (a.lmax + 1) * (a.lmax + 1) * N;
+    for (int64_t i = a.slot_offset[c]; i < a.slot_offset[c + 1]; i++) {
+        const PsKeySlot slot = a.slots[i];
+        const int64_t src = c * a.n_species + slot.a;
+        for (int k = threadIdx.x; k < K; k += blockDim.x) {
+            const int l = l_of_lm(k / N), width = (2 * l + 1) * N, w = k - l * l * N, blk = slot.block + l;
+            a.out[a.off_values[blk] + (int64_t)slot.sample * width + w] = a.coef[src * K + k];
+            if (do_strain) {
+                double* o = a.out + a.off_strain[blk] + (int64_t)slot.sample * 9 * width + w;
+                for (int x = 0; x < 9; x++) o[x * width] = a.strain[(src * 9 + x) * K + k];
+            }
+            if (do_cell) {
+                double* o = a.out + a.off_cell[blk] + (int64_t)slot.sample * 9 * width + w;
+                for (int x = 0; x < 9; x++) o[x * width] = a.cellg[(src * 9 + x) * K + k];
+            }
         }
     }
 }
 
-// positions gradient rows: self gradient for the centre, sum over the pairs
-// between centre and neighbour otherwise (spherical_expansion.rs:468-521)
-__global__ void se_output_gradients_kernel(SeOutArgs a) {
-    const int64_t row = blockIdx.x;
-    const int K = (a.lmax + 1) * (a.lmax + 1) * a.nmax;
-    const int blk = a.grad_block[row];
-    const int l = a.block_l[blk];
-    const int t = a.block_species[blk];
-    const int c = a.grad_centre[row];
-    const int j = a.grad_atom[row];
-    const int width = (2 * l + 1) * a.nmax;
-    const int start = l * l * a.nmax;
-    const double sign_l = (l & 1) ? -1.0 : 1.0;
-    double* out = a.out + a.off_positions[blk] + a.grad_row[row] * 3 * width;
-    for (int q = threadIdx.x; q < 3 * width; q += blockDim.x) {
-        int x = q / width, w = q - x * width;
-        double v;
-        if (c == j) {
-            v = a.self_grad[(((int64_t)c * a.n_species + t) * 3 + x) * K + start + w];
-        } else {
-            v = 0.0;
-            for (int d = a.grad_d0[row]; d < a.grad_d1[row]; d++) {
-                int32_t code = a.dir_code[d];
-                int64_t p = code >> 1;
-                double factor = (code & 1) ? -sign_l : 1.0;
-                v += factor * a.pair_grad[(p * 3 + x) * K + start + w];
+// positions gradient rows (spherical_expansion.rs:468-521): for every
+// neighbour entry of a centre (and the centre itself) the rows of all l at
+// once, from the pairs' gradients (or the centre's own).  SE_SPLIT CTAs share
+// a centre's entries.  Bound by the memory stream: a row set is 3 (l m n)
+// doubles read and written.  Row numbers come from the neighbourhood tables
+// on the device: the list of rows that the host used to make and upload (7
+// per entry) was 6 of the 7.3 ms of a call on 500 atoms (1.4 now), and one CTA
+// per row of 24 to 312 doubles took 358 us where this takes 165 (340 MB
+// written, 164 read: 3.1 TB/s).
+constexpr int SE_SPLIT = 4;
+
+__global__ void __launch_bounds__(256) se_output_gradients_kernel(SeOutArgs a) {
+    extern __shared__ int se_l[];  // [K] l of every coefficient
+    __shared__ int slot_of[64];    // slot of every species, -1: none
+    const int64_t c = blockIdx.x / SE_SPLIT;
+    const int part = (int)(blockIdx.x - c * SE_SPLIT);
+    const int N = a.nmax, K = (a.lmax + 1) * (a.lmax + 1) * N, S = a.n_species;
+    const int64_t s0 = a.slot_offset[c], s1 = a.slot_offset[c + 1];
+    for (int k = threadIdx.x; k < K; k += blockDim.x) se_l[k] = l_of_lm(k / N);
+    if (threadIdx.x < 64) slot_of[threadIdx.x] = -1;
+    __syncthreads();
+    for (int64_t i = s0 + threadIdx.x; i < s1; i += blockDim.x) slot_of[a.slots[i].a] = (int)(i - s0);
+    __syncthreads();
+    const int64_t e0 = a.entry_offset[c], n = a.entry_offset[c + 1] - e0;
+    const int64_t ee = e0 + n * (part + 1) / SE_SPLIT;
+    for (int64_t e = e0 + n * part / SE_SPLIT; e < ee; e++) {
+        const PsEntry entry = a.entries[e];
+        const bool self = entry.atom == (int32_t)c;
+        const int first = self ? 0 : slot_of[entry.species], last = self ? (int)(s1 - s0) : first + 1;
+        for (int i = first; i < last; i++) {
+            if (i < 0) continue;
+            const PsKeySlot slot = a.slots[s0 + i];
+            const int32_t* cum = a.entry_cum + e * (S + 1);
+            const int64_t row = a.slot_row[s0 + i] + cum[slot.a] + cum[S];
+            const double* own = self ? a.self_grad + (c * S + slot.a) * 3 * K : nullptr;
+            const int32_t code0 = self ? 0 : a.dir_code[entry.d0];
+            const bool single = entry.d1 - entry.d0 == 1;
+            for (int k = threadIdx.x; k < K; k += blockDim.x) {
+                const int l = se_l[k], width = (2 * l + 1) * N;
+                const double sign_l = (l & 1) ? -1.0 : 1.0;
+                double* o = a.out + a.off_positions[slot.block + l] + row * 3 * width + (k - l * l * N);
+                double v[3];
+                if (self) {
+#pragma unroll
+                    for (int x = 0; x < 3; x++) v[x] = own[x * K + k];
+                } else if (single) {
+                    const double* g = a.pair_grad + (int64_t)(code0 >> 1) * 3 * K + k;
+                    const double factor = (code0 & 1) ? -sign_l : 1.0;
+#pragma unroll
+                    for (int x = 0; x < 3; x++) v[x] = 0.0 + factor * g[x * K];
+                } else {
+                    v[0] = v[1] = v[2] = 0.0;
+                    for (int d = entry.d0; d < entry.d1; d++) {
+                        const int32_t code = a.dir_code[d];
+                        const double* g = a.pair_grad + (int64_t)(code >> 1) * 3 * K + k;
+                        const double factor = (code & 1) ? -sign_l : 1.0;
+#pragma unroll
+                        for (int x = 0; x < 3; x++) v[x] += factor * g[x * K];
+                    }
+                }
+#pragma unroll
+                for (int x = 0; x < 3; x++) __stcs(o + x * width, v[x]);
             }
         }
-        out[q] = v;
     }
 }
 
@@ -718,12 +754,14 @@ void launch_by_pair(const ByPairArgs& args, bool positions, bool strain, bool ce
 }
 
 void launch_se_output(const SeOutArgs& args, bool positions, bool strain, bool cell, cudaStream_t stream) {
-    if (args.n_rows > 0) {
-        se_output_rows_kernel<<<(unsigned)args.n_rows, 128, 0, stream>>>(args, strain, cell);
-        CUDA_CHECK(cudaGetLastError());
-    }
-    if (positions && args.n_grad_rows > 0) {
-        se_output_gradients_kernel<<<(unsigned)args.n_grad_rows, 128, 0, stream>>>(args);
+    if (args.n_centres == 0) return;
+    se_output_rows_kernel<<<(unsigned)args.n_centres, 128, 0, stream>>>(args, strain, cell);
+    CUDA_CHECK(cudaGetLastError());
+    if (positions) {
+        const size_t smem = sizeof(int) * (size_t)(args.lmax + 1) * (args.lmax + 1) * args.nmax;
+        if (smem > 48 * 1024)
+            CUDA_CHECK(cudaFuncSetAttribute(se_output_gradients_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        se_output_gradients_kernel<<<(unsigned)(args.n_centres * SE_SPLIT), 256, smem, stream>>>(args);
         CUDA_CHECK(cudaGetLastError());
     }
 }

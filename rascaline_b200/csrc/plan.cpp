@@ -351,8 +351,9 @@ OutputPlan plan_spherical_expansion(const Neighborhoods& nh, const Hypers& h, co
     OutputPlan plan;
     const int S = nh.n_species;
     const int L = h.max_angular;
+    const int64_t N = nh.n_atoms;
     std::vector<uint8_t> present((size_t)S * S, 0);
-    for (int64_t c = 0; c < nh.n_atoms; c++)
+    for (int64_t c = 0; c < N; c++)
         for (int t = 0; t < S; t++)
             if (nh.species_mask[(size_t)c * S + t]) present[(size_t)nh.atom_species[c] * S + t] = 1;
     // keys: (l, 1, center, neighbor) with l varying fastest
@@ -366,44 +367,87 @@ OutputPlan plan_spherical_expansion(const Neighborhoods& nh, const Hypers& h, co
                 plan.keys.values.insert(plan.keys.values.end(), {l, 1, nh.species_types[ct], nh.species_types[nt]});
                 plan.blocks.emplace_back();
                 plan.blocks.back().l = l;
-                plan.blocks.back().species = nt;
-                plan.blocks.back().samples.names = {"system", "atom"};
-                plan.blocks.back().gradient_samples.names = {"sample", "system", "atom"};
-                plan.block_l.push_back(l);
-                plan.block_species.push_back(nt);
             }
         }
-    for (int64_t c = 0; c < nh.n_atoms; c++) {
+    // slots, sample rows and the first gradient row of every slot: the rows of
+    // a (centre type, neighbour type) are the same for every l
+    plan.slot_offset.assign(N + 1, 0);
+    for (int64_t c = 0; c < N; c++) {
         for (int nt = 0; nt < S; nt++) {
             if (!nh.species_mask[(size_t)c * S + nt]) continue;
-            int32_t b0 = pair_block[(size_t)nh.atom_species[c] * S + nt];
-            for (int l = 0; l <= L; l++) {
-                auto& bp = plan.blocks[b0 + l];
-                int32_t sample = (int32_t)bp.n_samples++;
-                bp.samples.values.insert(bp.samples.values.end(), {nh.atom_system[c], nh.atom_local[c]});
-                plan.row_centre.push_back((int32_t)c);
-                plan.row_block.push_back(b0 + l);
-                plan.row_sample.push_back(sample);
-                if (!g.positions) continue;
-                for (int64_t e = nh.entry_offset[c]; e < nh.entry_offset[c + 1]; e++) {
-                    const PsEntry& en = nh.entries[e];
-                    if (en.atom != (int32_t)c && en.species != nt) continue;
-                    plan.grad_block.push_back(b0 + l);
-                    plan.grad_row.push_back(bp.n_grad_rows++);
-                    plan.grad_centre.push_back((int32_t)c);
-                    plan.grad_atom.push_back(en.atom);
-                    plan.grad_d0.push_back(en.d0);
-                    plan.grad_d1.push_back(en.d1);
-                    bp.gradient_samples.values.insert(bp.gradient_samples.values.end(),
-                                                      {sample, nh.atom_system[c], nh.atom_local[en.atom]});
+            const int32_t b0 = pair_block[(size_t)nh.atom_species[c] * S + nt];
+            auto& bp = plan.blocks[b0];
+            plan.slots.push_back(PsKeySlot{b0, (int32_t)bp.n_samples++, nt, nt});
+            plan.slot_row.push_back(bp.n_grad_rows);
+            if (g.positions) bp.n_grad_rows += nh.species_count[(size_t)c * S + nt] + 1;
+        }
+        plan.slot_offset[c + 1] = (int64_t)plan.slots.size();
+    }
+    std::vector<int64_t> widths;
+    for (size_t b = 0; b < plan.blocks.size(); b++) {
+        auto& bp = plan.blocks[b];
+        const auto& first = plan.blocks[b - bp.l];
+        bp.n_samples = first.n_samples;
+        bp.n_grad_rows = first.n_grad_rows;
+        widths.push_back((int64_t)(2 * bp.l + 1) * h.nmax());
+    }
+    assign_offsets(plan, g, widths);
+    return plan;
+}
+
+void fill_spherical_expansion_labels(const Neighborhoods& nh, const GradientOptions& g, OutputPlan& plan) {
+    const int64_t N = nh.n_atoms;
+    const int S = nh.n_species;
+    const int64_t nb = (int64_t)plan.blocks.size();
+    // the labels of the l = 0 blocks, then copies for the other l
+    for (int64_t b = 0; b < nb; b++) {
+        auto& bp = plan.blocks[b];
+        bp.samples.names = {"system", "atom"};
+        bp.gradient_samples.names = {"sample", "system", "atom"};
+        if (bp.l != 0) continue;
+        bp.samples.values.resize((size_t)bp.n_samples * 2);
+        if (g.positions) bp.gradient_samples.values.resize((size_t)bp.n_grad_rows * 3);
+    }
+    const int threads = (int)std::max<int64_t>(1, std::min<int64_t>(omp_get_max_threads(), (int64_t)plan.slots.size() / 64));
+#pragma omp parallel num_threads(threads)
+    {
+        std::vector<int32_t*> w(S);
+#pragma omp for schedule(static)
+        for (int64_t c = 0; c < N; c++) {
+            const int32_t sys = nh.atom_system[c];
+            const int64_t s0 = plan.slot_offset[c], s1 = plan.slot_offset[c + 1];
+            std::fill(w.begin(), w.end(), nullptr);
+            for (int64_t i = s0; i < s1; i++) {
+                const PsKeySlot& slot = plan.slots[i];
+                auto& bp = plan.blocks[slot.block];
+                int32_t* sw = bp.samples.values.data() + 2 * (size_t)slot.sample;
+                sw[0] = sys;
+                sw[1] = nh.atom_local[c];
+                if (g.positions) w[slot.a] = bp.gradient_samples.values.data() + 3 * (size_t)plan.slot_row[i];
+            }
+            if (!g.positions) continue;
+            for (int64_t e = nh.entry_offset[c]; e < nh.entry_offset[c + 1]; e++) {
+                const PsEntry& en = nh.entries[e];
+                for (int64_t i = s0; i < s1; i++) {
+                    const PsKeySlot& slot = plan.slots[i];
+                    if (en.atom != (int32_t)c && en.species != slot.a) continue;
+                    int32_t*& gw = w[slot.a];
+                    gw[0] = slot.sample;
+                    gw[1] = sys;
+                    gw[2] = nh.atom_local[en.atom];
+                    gw += 3;
                 }
             }
         }
+#pragma omp for schedule(dynamic)
+        for (int64_t b = 0; b < nb; b++) {
+            auto& bp = plan.blocks[b];
+            if (bp.l == 0) continue;
+            const auto& first = plan.blocks[b - bp.l];
+            bp.samples.values = first.samples.values;
+            bp.gradient_samples.values = first.gradient_samples.values;
+        }
     }
-    std::vector<int64_t> widths;
-    for (auto& bp : plan.blocks) widths.push_back((int64_t)(2 * bp.l + 1) * h.nmax());
-    assign_offsets(plan, g, widths);
-    return plan;
 }
 
 // spherical_expansion_by_pair (spherical_expansion_pair.rs:547-700) with the

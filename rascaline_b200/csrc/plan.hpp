@@ -53,22 +53,18 @@ struct BlockPlan {
     int64_t n_samples = 0, n_grad_rows = 0;
     int64_t off_values = 0, off_positions = -1, off_strain = -1, off_cell = -1;
     int l = 0;        // spherical expansion blocks
-    int species = 0;  // neighbour species (spherical expansion)
 };
 
 struct OutputPlan {
     Labels keys;
     std::vector<BlockPlan> blocks;
     int64_t total_doubles = 0;
-    // power spectrum tables
+    // slots of every centre: a (neighbour species pair) block of the power
+    // spectrum, or the l = 0 block of a neighbour species (a == b) of the
+    // spherical expansion, whose l > 0 blocks follow with the same rows
     std::vector<int64_t> slot_offset;  // [n_atoms + 1]
     std::vector<PsKeySlot> slots;
     std::vector<int64_t> slot_row;     // first gradient row of every slot
-    // spherical expansion tables
-    std::vector<int32_t> row_centre, row_block, row_sample;
-    std::vector<int32_t> grad_block, grad_centre, grad_atom, grad_d0, grad_d1;
-    std::vector<int64_t> grad_row;
-    std::vector<int32_t> block_l, block_species;
     // spherical expansion by pair, per direction d = 2 pair + reversed: the
     // block of l = 0 of its type pair (block of l = block0 + l), its row in
     // the l = 0 and l > 0 blocks and its first positions gradient row; and
@@ -85,7 +81,9 @@ struct OutputPlan {
 OutputPlan plan_power_spectrum(const Neighborhoods& nh, const Hypers& h, const GradientOptions& g,
                                bool with_labels = true);
 void fill_power_spectrum_labels(const Neighborhoods& nh, const GradientOptions& g, OutputPlan& plan);
+// the tables and offsets only; the labels by fill_spherical_expansion_labels
 OutputPlan plan_spherical_expansion(const Neighborhoods& nh, const Hypers& h, const GradientOptions& g);
+void fill_spherical_expansion_labels(const Neighborhoods& nh, const GradientOptions& g, OutputPlan& plan);
 OutputPlan plan_by_pair(const Neighborhoods& nh, const Hypers& h, const GradientOptions& g, int64_t n_pairs,
                         const int32_t* first, const int32_t* second, const int32_t* shift);
 

@@ -961,10 +961,11 @@ __global__ void __launch_bounds__(128) ps_centre_rows_kernel(PsArgs a, int kinds
     }
     load_scales(L, scale_s);
     // the centre's entry among its neighbour entries (sorted by atom index)
-    const int64_t e0 = a.entry_offset[c], ne = a.entry_offset[c + 1] - e0;
+    const bool with_self = kinds & CR_SELF;  // the only rows that need the entries
+    const int64_t e0 = with_self ? a.entry_offset[c] : 0, ne = with_self ? a.entry_offset[c + 1] - e0 : 0;
     if (warp == 0) {
         int64_t found = -1;
-        if (kinds & CR_SELF) {
+        if (with_self) {
             for (int64_t base = 0; base < ne && found < 0; base += 32) {
                 const bool hit = base + lane < ne && a.entries[e0 + base + lane].atom == (int32_t)c;
                 const unsigned mask = __ballot_sync(0xffffffffu, hit);
@@ -1100,7 +1101,7 @@ void launch_all(const PsArgs& args, bool values, bool positions, bool strain, bo
     const bool staged = positions && dmma_rows && args.n_species <= STG_MAX_SPECIES && stg.bytes <= 200 * 1024;
     const size_t cr_bytes = sizeof(double) * ((size_t)args.n_species * 32 * stg_steps(args.lmax) + 2 * (args.lmax + 1));
     const int gradient_kinds = (staged ? CR_SELF : 0) | (strain ? CR_STRAIN : 0) | (cell ? CR_CELL : 0);
-    const bool centre_rows = dmma_rows && cr_bytes <= 200 * 1024 && gradient_kinds != 0 && (staged || !positions);
+    const bool centre_rows = dmma_rows && cr_bytes <= 200 * 1024 && (staged || !positions) && gradient_kinds != 0;
     const int kinds = gradient_kinds | (values ? CR_VALUES : 0);
     if (values && !centre_rows) {
         ps_values_kernel<MAXN><<<(unsigned)args.n_centres, threads, coef_bytes, side>>>(args);
@@ -1340,16 +1341,18 @@ __global__ void neighborhoods_count_kernel(const int32_t* __restrict__ first, co
 DeviceNeighborhoods launch_neighborhoods(const DevicePairs& pairs, const int32_t* atom_species, const int32_t* dir_code,
                                          const int64_t* seg_offset, int n_species, int64_t n_atoms, DeviceArena& arena,
                                          cudaStream_t stream, int32_t* host_count, uint8_t* host_mask,
-                                         cudaEvent_t counted) {
+                                         cudaEvent_t counted, bool with_entries) {
     if (n_species > NB_MAX_SPECIES) throw invalid_parameter("more than 64 atomic types are not supported");
     if (2 * pairs.count + n_atoms >= (int64_t)INT32_MAX) throw invalid_parameter("too many pairs");
     DeviceNeighborhoods nb;
     const int S = n_species;
     const int64_t capacity = 2 * pairs.count + n_atoms;  // every direction and every centre at most once
     int64_t* counts = arena.alloc<int64_t>("nb.counts", n_atoms + 1);
-    nb.entry_offset = arena.alloc<int64_t>("nb.entry_offset", n_atoms + 1);
-    nb.entries = arena.alloc<PsEntry>("nb.entries", capacity);
-    nb.entry_cum = arena.alloc<int32_t>("nb.entry_cum", capacity * (S + 1));
+    if (with_entries) {
+        nb.entry_offset = arena.alloc<int64_t>("nb.entry_offset", n_atoms + 1);
+        nb.entries = arena.alloc<PsEntry>("nb.entries", capacity);
+        nb.entry_cum = arena.alloc<int32_t>("nb.entry_cum", capacity * (S + 1));
+    }
     nb.species_count = arena.alloc<int32_t>("nb.species_count", n_atoms * S);
     nb.species_mask = arena.alloc<uint8_t>("nb.species_mask", n_atoms * S);
     const unsigned count_blocks = (unsigned)(((n_atoms + 1) * 32 + 255) / 256);
@@ -1363,6 +1366,7 @@ DeviceNeighborhoods launch_neighborhoods(const DevicePairs& pairs, const int32_t
         CUDA_CHECK(cudaMemcpyAsync(host_mask, nb.species_mask, n_atoms * S, cudaMemcpyDeviceToHost, stream));
         if (counted) CUDA_CHECK(cudaEventRecord(counted, stream));
     }
+    if (!with_entries) return nb;
     size_t temp = 0;
     CUDA_CHECK(cub::DeviceScan::ExclusiveSum(nullptr, temp, counts, nb.entry_offset, (int)(n_atoms + 1), stream));
     void* scan_temp = arena.alloc_bytes("nb.scan_temp", temp);  // its own: this may run beside other scans
