@@ -260,7 +260,7 @@ def dense_rooflines(phases, n_atoms, S, K, n_keys, n_props, grad_rows, peak, pea
     for name, phase, bytes_ in (("contraction", "contraction", contraction), ("dl_dc", "dl_dc", grad)):
         ms = phases.get(phase, 0.0)
         achieved = bytes_ / (ms / 1e3) / 1e9 if ms > 0 else 0.0
-        out[name] = {"kernel": "dense_contraction_mma" if name == "contraction" else "dense_grad_coef_mma",
+        out[name] = {"kernel": "dense_contraction_tiles" if name == "contraction" else "dense_grad_coef_mma",
                      "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "peak_source": peak_kind, "algorithmic_bytes_per_launch": bytes_,
                      "time_ms": ms}

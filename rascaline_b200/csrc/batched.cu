@@ -108,6 +108,13 @@ BatchPlan::BatchPlan(Engine& engine, const std::vector<int64_t>& sizes, const st
     d_atom_offset_ = (int64_t*)put(atom_offset.data(), 8 * atom_offset.size());
     d_h_offset_ = (int64_t*)put(h_offset.data(), 8 * h_offset.size());
     d_order_ = (int32_t*)put(order.data(), 4 * order.size());
+    {
+        std::vector<int32_t> by_species;
+        const std::vector<int32_t> tiles = dense_species_tiles(sp, S, by_species);
+        n_species_tiles_ = (int)(tiles.size() / 3);
+        d_species_order_ = (int32_t*)put(by_species.data(), 4 * by_species.size());
+        d_species_tiles_ = (int32_t*)put(tiles.data(), 4 * tiles.size());
+    }
     d_control_ = (int32_t*)put(nullptr, 64);
     d_h_ = (float*)put(nullptr, sizeof(float) * 3 * (size_t)std::max<int64_t>(hsum, 1));
     d_atom_energy_ = (float*)put(nullptr, sizeof(float) * (size_t)std::max<int64_t>(n_atoms_, 1));
@@ -178,20 +185,29 @@ void BatchPlan::run_dense(const double* positions, const float* weights, const f
         vals = d_values_scratch_;
     }
     const bool backward = (weights || grad_values) && (grad_positions || grad_strain);
+    SpeciesModel model;
+    model.weights = energies ? weights : nullptr;
+    model.atom_energy = d_atom_energy_;
+    model.order = d_species_order_;
+    model.tiles = d_species_tiles_;
+    model.n_tiles = n_species_tiles_;
     auto st = engine_.forward_dense(32, systems_, positions, species_, vals, n_atoms_ * kp, stream,
-                                    /*expansion=*/false, /*backward_follows=*/backward);
+                                    /*expansion=*/false, /*backward_follows=*/backward, &model);
     if (backward) {
         float* gp = grad_positions;
         if (!gp) {
             if (!d_grad_scratch_) CUDA_CHECK(cudaMalloc(&d_grad_scratch_, sizeof(float) * 3 * (size_t)n_atoms_));
             gp = d_grad_scratch_;
         }
-        if (weights) engine_.backward_dense(*st, weights, gp, grad_strain, nullptr, stream, /*by_species=*/true);
+        if (weights) engine_.backward_dense(*st, weights, gp, grad_strain, nullptr, stream, /*by_species=*/true,
+                                             /*coefficients=*/false, &model);
         else engine_.backward_dense(*st, grad_values, gp, grad_strain, nullptr, stream);
     }
     if (energies && weights) {
-        batch_atom_energy<<<(unsigned)n_atoms_, 256, 0, stream>>>(vals, weights, d_species_, kp, d_atom_energy_);
-        CUDA_CHECK(cudaGetLastError());
+        if (!st->energies) {
+            batch_atom_energy<<<(unsigned)n_atoms_, 256, 0, stream>>>(vals, weights, d_species_, kp, d_atom_energy_);
+            CUDA_CHECK(cudaGetLastError());
+        }
         const int64_t ns = (int64_t)sizes_.size();
         batch_system_energy<<<(unsigned)((ns + 127) / 128), 128, 0, stream>>>(d_atom_energy_, d_atom_offset_, ns,
                                                                               energies);

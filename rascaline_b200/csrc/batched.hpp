@@ -112,6 +112,10 @@ class BatchPlan {
     int64_t* d_atom_offset_ = nullptr;
     int64_t* d_h_offset_ = nullptr;
     int32_t* d_order_ = nullptr;
+    // dense pipeline: the atoms by species and their tiles
+    int32_t* d_species_order_ = nullptr;
+    int32_t* d_species_tiles_ = nullptr;
+    int n_species_tiles_ = 0;
     int32_t* d_control_ = nullptr;  // queue, barrier (2), status
     float* d_h_ = nullptr;
     float* d_atom_energy_ = nullptr;

@@ -889,12 +889,10 @@ void launch_dense_forward(const DenseArgs<T>& a, int64_t n_pairs, cudaStream_t s
         mark(3);
         return;
     }
-    if constexpr (sizeof(T) == 4) {
-        if (dense_mma_enabled() && dense_mma_supported(a)) {
-            launch_dense_contraction_mma(a, stream);
-            mark(3);
-            return;
-        }
+    if (dense_contraction_by_warp(a)) {
+        launch_dense_contraction_warp(a, stream);
+        mark(3);
+        return;
     }
     const size_t smem = sizeof(T) * (size_t)a.n_species * a.K;
     if (a.nmax <= 16 && smem <= 48 * 1024) {
@@ -924,7 +922,17 @@ void launch_dense_grad_coef(const DenseArgs<T>& a, cudaStream_t stream) {
     const size_t tiled_smem = smem + sizeof(T) * (size_t)a.n_keys * a.n_props;
     bool mma = false;
     if constexpr (sizeof(T) == 4) mma = dense_mma_enabled() && dense_mma_supported(a);
-    if (mma) {
+    if constexpr (sizeof(T) == 8) {
+        if (dense_grad_coef_by_warp(a)) {
+            launch_dense_grad_coef_warp(a, stream);
+            return;
+        }
+    }
+    bool by_species = false;
+    if constexpr (sizeof(T) == 4) by_species = dense_mma_enabled() && dense_grad_coef_species_supported(a);
+    if (by_species) {
+        if constexpr (sizeof(T) == 4) launch_dense_grad_coef_species(a, stream);
+    } else if (mma) {
         if constexpr (sizeof(T) == 4) launch_dense_grad_coef_mma(a, stream);
     } else if (a.lmax <= DENSE_LMAX_SMALL && tiled_smem <= 200 * 1024) {
         dense_grad_coef_tiled<T, 17><<<(unsigned)a.n_atoms, 128, tiled_smem, stream>>>(a);

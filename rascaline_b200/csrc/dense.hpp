@@ -42,6 +42,15 @@ struct DenseArgs {
     // when set, the dL/dP row of centre c is grad_values[grad_species[c]]:
     // one row per species (the weights of a linear model)
     const int32_t* grad_species = nullptr;
+    // with grad_species: the atoms sorted by species, and (species, first,
+    // count) of the tiles that share one left operand (dense_warp.cu)
+    const int32_t* species_order = nullptr;
+    const int32_t* species_tiles = nullptr;
+    int n_species_tiles = 0;
+    // forward: with weights [species][keys][props], each atom's sum of
+    // weights x values
+    const T* energy_weights = nullptr;
+    T* energy = nullptr;
     T* grad_coef;         // [n_atoms][S][K]
     T* pair_grad;         // [n_pairs][3] dL/dr_ij
     T* grad_positions;    // [n_atoms][3]
@@ -85,6 +94,8 @@ struct DenseState {
     // the caller announced a backward pass that recomputes them otherwise
     // (FP32 with the learned radial surrogate); the backward reads them
     void* features_grad = nullptr;
+    // the forward pass computed the atoms' energies of its SpeciesModel
+    bool energies = false;
 
     DenseState() = default;
     DenseState(const DenseState&) = delete;
@@ -95,10 +106,9 @@ struct DenseState {
     std::vector<void*> allocations_;
 };
 
-// FP32 contractions on the tensor cores (dense_mma.cu): the power spectrum
-// P_l = X_l^T X_l and dL/dc; supported when S nmax <= 128 and 2 lmax + 1 <= 32
+// FP32 dL/dc on the tcgen05 tensor cores (dense_mma.cu), supported when
+// S nmax <= 128 and 2 lmax + 1 <= 32
 bool dense_mma_supported(const DenseArgs<float>& a);
-void launch_dense_contraction_mma(const DenseArgs<float>& a, cudaStream_t stream);
 void launch_dense_grad_coef_mma(const DenseArgs<float>& a, cudaStream_t stream);
 // angular channels per round of the tensor-core kernels (1 to 4)
 extern int dense_mma_channels_per_round;
@@ -106,6 +116,29 @@ extern int dense_mma_channels_per_round;
 // cores; FEATOMIC_B200_DENSE_MMA=0 in the environment selects the CUDA cores
 bool dense_mma_enabled();
 void set_dense_mma_enabled(bool enabled);
+
+// the same with a warp per centre (dense_warp.cu): the power spectrum (and
+// the energies, when a.energy is set), and dL/dc for rows of dL/dP by species
+template <typename T>
+bool dense_contraction_by_warp(const DenseArgs<T>& a);
+template <typename T>
+void launch_dense_contraction_warp(const DenseArgs<T>& a, cudaStream_t stream);
+bool dense_grad_coef_by_warp(const DenseArgs<double>& a);
+void launch_dense_grad_coef_warp(const DenseArgs<double>& a, cudaStream_t stream);
+bool dense_grad_coef_species_supported(const DenseArgs<float>& a);
+void launch_dense_grad_coef_species(const DenseArgs<float>& a, cudaStream_t stream);
+// tiles (species, first, count) over `order`, the atoms sorted by species
+std::vector<int32_t> dense_species_tiles(const std::vector<int32_t>& species, int n_species, std::vector<int32_t>& order);
+
+// What a batch of systems adds to a forward and backward pass of a linear
+// model: one row of weights per species
+struct SpeciesModel {
+    const float* weights = nullptr;  // [species][keys][props]
+    float* atom_energy = nullptr;    // [n_atoms]
+    const int32_t* order = nullptr;
+    const int32_t* tiles = nullptr;
+    int n_tiles = 0;
+};
 
 template <typename T>
 void launch_dense_forward(const DenseArgs<T>& a, int64_t n_pairs, cudaStream_t stream);

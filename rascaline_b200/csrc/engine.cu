@@ -1049,7 +1049,7 @@ void Engine::dense_args(const DenseState& st, bool grad, DenseArgs<T>& a) {
 std::unique_ptr<DenseState> Engine::forward_dense(int precision, std::vector<HostSystem>& systems,
                                                   const double* d_positions, const std::vector<int32_t>& species,
                                                   void* values, int64_t values_count, cudaStream_t stream,
-                                                  bool expansion, bool backward_follows) {
+                                                  bool expansion, bool backward_follows, const SpeciesModel* model) {
     if (precision != 32 && precision != 64) throw invalid_parameter("precision must be 32 or 64");
     upload_tables();
     const std::shared_ptr<RadialSurrogate> hold = surrogate_.lock();
@@ -1161,6 +1161,11 @@ std::unique_ptr<DenseState> Engine::forward_dense(int precision, std::vector<Hos
         a.features = (float*)features;
         a.values = expansion ? nullptr : (float*)values;
         a.status = status;
+        if (model && model->weights && model->atom_energy && !expansion && dense_contraction_by_warp(a)) {
+            a.energy_weights = model->weights;
+            a.energy = model->atom_energy;
+            st->energies = true;
+        }
         launch_dense_forward<float>(a, P, stream);
     }
     if (expansion) {
@@ -1216,7 +1221,8 @@ void Engine::jvp_dense(DenseState& st, const void* tangent_positions, const void
 }
 
 void Engine::backward_dense(DenseState& st, const void* grad_values, void* grad_positions, void* grad_strain,
-                            void* grad_cell, cudaStream_t stream, bool by_species, bool coefficients) {
+                            void* grad_cell, cudaStream_t stream, bool by_species, bool coefficients,
+                            const SpeciesModel* model) {
     int dev = -1;
     CUDA_CHECK(cudaGetDevice(&dev));
     if (dev != st.device) throw invalid_parameter("the backward pass must run on the device of the forward pass");
@@ -1265,6 +1271,11 @@ void Engine::backward_dense(DenseState& st, const void* grad_values, void* grad_
         a.features = (float*)features;
         a.grad_values = (const float*)grad_values;
         a.grad_species = by_species ? st.atom_species : nullptr;
+        if (by_species && model) {
+            a.species_order = model->order;
+            a.species_tiles = model->tiles;
+            a.n_species_tiles = model->n_tiles;
+        }
         a.grad_coef = (float*)grad_coef;
         a.pair_grad = (float*)pair_grad;
         a.atom_partial = (float*)partial;

@@ -356,6 +356,7 @@ void launch_by_pair(const ByPairArgs& args, bool positions, bool strain, bool ce
 namespace fb200 {
 
 struct DenseState;
+struct SpeciesModel;
 struct Neighborhoods;
 template <typename T>
 struct DenseArgs;
@@ -395,7 +396,8 @@ class Engine {
     std::unique_ptr<DenseState> forward_dense(int precision, std::vector<HostSystem>& systems,
                                               const double* d_positions, const std::vector<int32_t>& species,
                                               void* values, int64_t values_count, cudaStream_t stream,
-                                              bool expansion = false, bool backward_follows = false);
+                                              bool expansion = false, bool backward_follows = false,
+                                              const SpeciesModel* model = nullptr);
     // dL/dpositions [n_atoms][3], and when not null dL/dstrain and dL/dcell
     // [n_systems][3][3], all device buffers of the forward precision
     // `by_species`: grad_values holds one dL/dP row per species (the weights
@@ -403,7 +405,8 @@ class Engine {
     // `coefficients`: grad_values is dL/dc [n_atoms][n_species][K] of the
     // spherical expansion instead of dL/dP
     void backward_dense(DenseState& state, const void* grad_values, void* grad_positions, void* grad_strain,
-                        void* grad_cell, cudaStream_t stream, bool by_species = false, bool coefficients = false);
+                        void* grad_cell, cudaStream_t stream, bool by_species = false, bool coefficients = false,
+                        const SpeciesModel* model = nullptr);
     // forward-mode derivative along a displacement of the positions
     // ([n_atoms][3]) and cells ([n_systems][3][3] or null): the tangent of the
     // coefficients (when `tangent_coef` is not null) and of the power spectrum

@@ -1,0 +1,108 @@
+"""Warp-per-centre contractions of the dense forms at the edges of their
+tiles: one to six species (four are the most that are known at compile time),
+one to forty radial functions (odd, fewer and more than eight, across blocks
+of 32), l up to 8, one centre and more than a CTA holds.
+
+* values and dL/dpositions, FP32 against the CUDA-core kernels: 2e-6 of the
+  largest value, the bound of the tensor-core kernels (TF32 hi + lo drops
+  2^-22 of a product; sums of at most 17 x 40 products);
+* FP64 values against the contraction in torch, and the FP64 gradient against
+  the transposed forward-mode derivative <G, J u> = <J^T G, u>: 1e-12 of the
+  sum of sizes (rounding of 1e3-term sums, 1e-16 each, with a factor 10);
+* a batch with weights by species against the same batch with every atom's
+  row given: 2e-6 on gradients, 1e-5 on energies (FP32 sums of 4480 terms).
+"""
+import numpy as np
+import pytest
+
+import rascaline_b200 as rb
+from rascaline_b200 import _c_api as C
+from rascaline_b200 import workloads
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+
+from rascaline_b200 import torch_api  # noqa: E402
+
+TYPES = (1, 6, 7, 8, 9, 16)
+
+
+@pytest.fixture(autouse=True)
+def restore_engine():
+    yield
+    C.check(C.lib().featomic_b200_set_contraction_engine(1, 1))
+
+
+def _forward(calculator, system, precision):
+    positions = torch.tensor(system["positions"], device="cuda")
+    cell = np.asarray(system["cell"]).reshape(1, 9)
+    return torch_api.dense_power_spectrum(calculator, positions, system["types"], cell, [len(system["types"])], precision)
+
+
+@pytest.mark.parametrize("atoms,species,max_radial,max_angular", [
+    (1, 1, 0, 0), (9, 1, 7, 8), (20, 2, 2, 3), (33, 3, 5, 6), (40, 4, 7, 6), (40, 4, 4, 5), (30, 6, 7, 2),
+    (20, 3, 11, 4), (12, 1, 15, 3),
+])
+def test_values_and_gradients(atoms, species, max_radial, max_angular):
+    if atoms > 1:
+        system = workloads.random_box(atoms, seed=atoms, species=TYPES[:species])
+    else:
+        system = workloads.system_dict([1], [[0.1, 0.2, 0.3]], np.zeros((3, 3)))
+    hypers = workloads.hypers(4.0, max_radial, max_angular)
+    calculator = rb.SoapPowerSpectrum(**hypers)
+    results = []
+    for engine in (1, 0):
+        C.check(C.lib().featomic_b200_set_contraction_engine(engine, 1))
+        values, state = _forward(calculator, system, 32)
+        gradient = torch.randn(values.shape, generator=torch.Generator().manual_seed(3)).cuda()
+        results.append([values] + [x for x in torch_api.dense_backward(state, gradient, 1) if x is not None])
+    for a, b in zip(*results):
+        assert float((a - b).abs().max()) <= 2e-6 * max(float(b.abs().max()), 1e-30)
+
+    values, state = _forward(calculator, system, 64)
+    positions = torch.tensor(system["positions"], device="cuda")
+    c, _ = torch_api.dense_spherical_expansion(rb.SphericalExpansion(**hypers), positions, system["types"],
+                                               np.asarray(system["cell"]).reshape(1, 9), [atoms], 64)
+    N, S = max_radial + 1, c.shape[1]
+    c = c.reshape(atoms, S, (max_angular + 1) ** 2, N)
+    key = 0
+    for a in range(S):
+        for b in range(a, S):
+            for l in range(max_angular + 1):
+                x, y = (c[:, s, l * l:(l + 1) ** 2] for s in (a, b))
+                scale = (-1) ** l / np.sqrt(2 * l + 1) * (np.sqrt(2) if a != b else 1)
+                reference = torch.einsum("cmp,cmq->cpq", x, y).reshape(atoms, -1) * scale
+                size = torch.einsum("cmp,cmq->cpq", x.abs(), y.abs()).reshape(atoms, -1) * abs(scale)
+                found = values[:, key, l * N * N:(l + 1) * N * N]
+                assert bool(((found - reference).abs() <= 1e-12 * size + 1e-300).all())
+            key += 1
+    gradient = torch.randn(values.shape, generator=torch.Generator().manual_seed(4), dtype=torch.float64).cuda()
+    move = torch.randn((atoms, 3), generator=torch.Generator().manual_seed(5), dtype=torch.float64).cuda()
+    forces, _, _ = torch_api.dense_backward(state, gradient, 1, cell=False)
+    tangent, _ = torch_api.dense_jvp(state, move)
+    size = float((gradient.abs() * tangent.abs()).sum())
+    assert abs(float((gradient * tangent).sum() - (forces * move).sum())) <= 1e-12 * size + 1e-300
+
+
+@pytest.mark.parametrize("molecules,species,max_radial,max_angular", [(1, 1, 1, 2), (12, 2, 7, 4), (40, 4, 7, 6), (9, 4, 4, 3)])
+def test_batch_weights_by_species(molecules, species, max_radial, max_angular):
+    systems = workloads.molecules(molecules, seed=5)
+    sizes = [len(m["types"]) for m in systems]
+    rng = np.random.default_rng(6)
+    types = rng.choice(TYPES[:species], size=sum(sizes)).astype(np.int32)
+    positions = torch.tensor(np.concatenate([m["positions"] for m in systems]), device="cuda")
+    batch = torch_api.Batch(rb.SoapPowerSpectrum(**workloads.hypers(4.5, max_radial, max_angular)), sizes, types,
+                            TYPES[:species])
+    batch.config = dict(batch.config, pipeline=1)
+    weights = torch.tensor(rng.normal(size=(species, batch.n_keys, batch.n_properties)), dtype=torch.float32, device="cuda")
+    out = batch.run(positions, batch.outputs(strain=True), weights=weights)
+    rows = weights[torch.tensor(np.searchsorted(TYPES[:species], types), device="cuda")].contiguous()
+    given = batch.run(positions, batch.outputs(energies=False, strain=True), grad_values=rows)
+    assert torch.equal(out["values"], given["values"])
+    for name in ("gradients", "strain"):
+        assert float((out[name] - given[name]).abs().max()) <= 2e-6 * float(given[name].abs().max())
+    per_atom = (given["values"].double() * rows.double()).flatten(1)
+    energies = torch.stack([x.sum() for x in torch.split(per_atom, sizes)])
+    size = torch.stack([x.abs().sum() for x in torch.split(per_atom, sizes)])
+    assert bool(((out["energies"] - energies).abs() <= 1e-5 * size).all())
