@@ -230,6 +230,13 @@ __global__ void __launch_bounds__(256) se_accumulate_kernel(SeArgs a) {
 // per (direction, l) the radial integral R_nl (+ dR/dr), one thread per
 // direction the cutoff and radial scaling; then every thread accumulates two
 // radial functions of one (l, m) over the chunk's directions in pair order.
+// Channels with the same knots share a direction's interval and weights, and
+// its spline rows are read by a thread per (l, n); products that do not depend
+// on (l, m, n) are made once per direction, signs are flipped instead of
+// multiplied, and a thread's two coefficients move as 16 bytes: 1000 atoms with
+// positions and strain 342 -> 278 us, 500 with positions 185 -> 152.  Bound by
+// the FP64 instructions (about 45 per coefficient and direction) at 14 warps
+// per SM.
 // The same functions in the same order as the two-kernel path, so the results
 // are bit-identical to it; no atomics.
 constexpr int FUSED_CHUNK = 32;
@@ -239,19 +246,46 @@ struct FusedDir {
     // f R dY / r is evaluated as f R dY * rinv (one extra rounding against
     // featomic's division, far inside the 1e-10 parity bound; an FP64 divide
     // per coefficient was most of this kernel's instruction stream)
-    double f, fg, r, rinv, u[3], v[3], sh[3];
+    // fgu = f' u; v and sh with the sign of the direction
+    double f, rinv, fgu[3], u[3], v[3], sh[3];
     int64_t pair;
     int inv, self_image;
 };
 
-__host__ __device__ inline size_t fused_shared_doubles(int lmax, int nmax, bool grad) {
+// two coefficients (n, n + 1) of a row: 16 bytes at once when n + 1 exists and
+// rows are even
+__device__ __forceinline__ void load_two(const double* p, bool even, double (&v)[2]) {
+    if (even) {
+        const double2 w = *reinterpret_cast<const double2*>(p);
+        v[0] = w.x;
+        v[1] = w.y;
+    } else {
+        v[0] = p[0];
+        v[1] = p[1];
+    }
+}
+__device__ __forceinline__ void store_two(double* p, bool even, bool second, const double (&v)[2]) {
+    if (even) {
+        *reinterpret_cast<double2*>(p) = make_double2(v[0], v[1]);
+    } else {
+        p[0] = v[0];
+        if (second) p[1] = v[1];
+    }
+}
+
+// Hermite weights of one (direction, level of knots): values, derivatives,
+// 1 / width
+constexpr int FUSED_WEIGHTS = 9;
+
+__host__ __device__ inline size_t fused_shared_doubles(int lmax, int nmax, bool grad, int levels) {
     const int L2 = (lmax + 1) * (lmax + 1), LR = (lmax + 1) * nmax, NP = (lmax + 1) * (lmax + 2) / 2;
-    return (size_t)FUSED_CHUNK * (L2 * (grad ? 4 : 1) + LR * (grad ? 2 : 1) + NP);
+    // ... and per (direction, level) the weights and the spline row
+    return (size_t)FUSED_CHUNK * (L2 * (grad ? 4 : 1) + LR * (grad ? 2 : 1) + NP + levels * (FUSED_WEIGHTS + 1));
 }
 
 template <bool POS, bool STRAIN, bool CELL>
 __global__ void __launch_bounds__(256, 2) se_fused_kernel(SeArgs a, DevicePairs pairs, DeviceRadial radial, DeviceYlm ylm,
-                                                        CutoffParams cut) {
+                                                        CutoffParams cut, DeviceSplineT<double> spline) {
     constexpr bool GRAD = POS || STRAIN || CELL;
     extern __shared__ double fsm[];
     __shared__ FusedDir dirs[FUSED_CHUNK];
@@ -262,6 +296,12 @@ __global__ void __launch_bounds__(256, 2) se_fused_kernel(SeArgs a, DevicePairs 
     double* Rs = dYs + (GRAD ? FUSED_CHUNK * 3 * L2 : 0);  // [chunk][LR]
     double* dRs = Rs + FUSED_CHUNK * LR;                   // [chunk][LR]
     double* Ps = dRs + (GRAD ? FUSED_CHUNK * LR : 0);      // [chunk][NP] Legendre table
+    // channels with the same knots share the interval and the weights; with
+    // more kinds of knots than the spline's levels hold, a thread per
+    // (direction, l) evaluates its own
+    const int levels = spline.levels;
+    double* Hs = Ps + FUSED_CHUNK * NP;                    // [chunk][levels][FUSED_WEIGHTS]
+    int* Ks = reinterpret_cast<int*>(Hs + FUSED_CHUNK * levels * FUSED_WEIGHTS);  // [chunk][levels]
     const int S = a.n_species;
     const int64_t c = blockIdx.x / S;
     const int t = (int)(blockIdx.x - c * S);
@@ -273,12 +313,13 @@ __global__ void __launch_bounds__(256, 2) se_fused_kernel(SeArgs a, DevicePairs 
     const bool active = item < L2 * NH;
     const int lm = active ? item / NH : 0;
     const int n0 = active ? 2 * (item - lm * NH) : 0;
-    const bool has1 = n0 + 1 < N;
+    const bool has1 = n0 + 1 < N, even = (N & 1) == 0;
     int l = (int)sqrt((double)lm);
     while (l * l > lm) l--;
     while ((l + 1) * (l + 1) <= lm) l++;
-    const double sign_l = (l & 1) ? -1.0 : 1.0;
-    const int ri = l * N + n0;
+    const bool odd_l = l & 1;
+    const double sign_l = odd_l ? -1.0 : 1.0;
+    const int ri = l * N + n0, k0 = lm * N + n0;
     double acc[2] = {0.0, 0.0};
     double sg[2][3], st[2][9], ce[2][9];
 #pragma unroll
@@ -296,15 +337,33 @@ __global__ void __launch_bounds__(256, 2) se_fused_kernel(SeArgs a, DevicePairs 
         const int lcols = L.lmax + 1;
         __syncthreads();
         // threads [0, nd * lcols): direction q, Legendre column m (the m = 0
-        // thread also writes the direction's scalars); threads
-        // [nd * lcols, 2 nd * lcols): direction q, radial channel l
-        for (int w = threadIdx.x; w < 2 * nd * lcols; w += blockDim.x) {
+        // thread also writes the direction's scalars); the threads after them:
+        // direction q, level of knots (or radial channel l)
+        const int rcols = levels > 0 ? levels : lcols;
+        for (int w = threadIdx.x; w < nd * (lcols + rcols); w += blockDim.x) {
             const bool column = w < nd * lcols;
-            const int wq = column ? w : w - nd * lcols;
-            const int q = wq / lcols, j = wq - q * lcols;
+            const int wq = column ? w : w - nd * lcols, cols = column ? lcols : rcols;
+            const int q = wq / cols, j = wq - q * cols;
             const int32_t code = a.dir_code[dc + q];
             const int64_t p = code >> 1;
             const double r = pairs.distance[p];
+            if (!column && levels > 0) {
+                double2 knot, next;
+                const int k = level_interval(spline, j, r, knot, next);
+                const soap::HermiteWeights h = soap::hermite_weights(knot.x, next.x, r);
+                double* o = Hs + (q * levels + j) * FUSED_WEIGHTS;
+                o[0] = h.h00;
+                o[1] = h.h10 * h.delta;
+                o[2] = h.h01;
+                o[3] = h.h11 * h.delta;
+                o[4] = h.d00;
+                o[5] = h.d10;
+                o[6] = h.d01;
+                o[7] = h.d11;
+                o[8] = h.dxdt;
+                Ks[q * levels + j] = k * spline.quad_pitch[j];
+                continue;
+            }
             if (!column) {
                 radial_spline_compute(radial, j, r, Rs + q * LR + j * N, GRAD ? dRs + q * LR + j * N : nullptr);
                 continue;
@@ -326,18 +385,24 @@ __global__ void __launch_bounds__(256, 2) se_fused_kernel(SeArgs a, DevicePairs 
             if (cut.scaling) soap::willatt2018(cut.scale, cut.rate, cut.exponent, r, &sc, &dsc);
             FusedDir& D = dirs[q];
             D.f = sc * fc;
-            D.fg = dfc * sc + fc * dsc;
-            D.r = r;
+            const double fg = dfc * sc + fc * dsc;
+            D.fgu[0] = fg * u0;
+            D.fgu[1] = fg * u1;
+            D.fgu[2] = fg * u2;
             D.rinv = 1.0 / r;
             D.u[0] = u0;
             D.u[1] = u1;
             D.u[2] = u2;
-            D.v[0] = v0;
-            D.v[1] = v1;
-            D.v[2] = v2;
-            for (int x = 0; x < 3; x++) D.sh[x] = (double)pairs.shift[3 * p + x];
+            const bool inv = code & 1;
+            D.v[0] = inv ? -v0 : v0;
+            D.v[1] = inv ? -v1 : v1;
+            D.v[2] = inv ? -v2 : v2;
+            for (int x = 0; x < 3; x++) {
+                const double sh = (double)pairs.shift[3 * p + x];
+                D.sh[x] = inv ? -sh : sh;
+            }
             D.pair = p;
-            D.inv = code & 1;
+            D.inv = inv;
             D.self_image = pairs.first[p] == pairs.second[p];
         }
         __syncthreads();
@@ -350,36 +415,59 @@ __global__ void __launch_bounds__(256, 2) se_fused_kernel(SeArgs a, DevicePairs 
             ylm_column_outputs(ylm, ylm_angles(D.u[0], D.u[1], D.u[2]), m, Ps + q * NP, Y, G,
                                GRAD ? G + L2 : nullptr, GRAD ? G + 2 * L2 : nullptr);
         }
+        // R_nl and dR/dr: a thread per (l, n) for every groups-th direction,
+        // whose loads of one direction are contiguous
+        if (levels > 0) {
+            const int groups = max(1, (int)blockDim.x / LR);
+            for (int w = threadIdx.x; w < groups * LR; w += blockDim.x) {
+                const int group = w / LR, ln = w - group * LR, lr = ln / N;
+                const int level = spline.level_of[lr];
+                const double* quads = spline.quads + 4 * (spline.first_quad[lr] + ln - lr * N);
+                for (int q = group; q < nd; q += groups) {
+                    const double* h = Hs + (q * levels + level) * FUSED_WEIGHTS;
+                    double x[4];
+                    load_quad_global(quads + 4 * Ks[q * levels + level], x);
+                    Rs[q * LR + ln] = h[0] * x[0] + h[1] * x[1] + h[2] * x[2] + h[3] * x[3];
+                    if (GRAD) dRs[q * LR + ln] = h[4] * x[0] * h[8] + h[5] * x[1] + h[6] * x[2] * h[8] + h[7] * x[3];
+                }
+            }
+        }
         __syncthreads();
         if (!active) continue;
         for (int q = 0; q < nd; q++) {
             const FusedDir& D = dirs[q];
             const double Yv = Ys[q * L2 + lm];
-            double dY[3] = {0.0, 0.0, 0.0};
+            double R[2], dR[2], dY[3];
+            load_two(Rs + q * LR + ri, even, R);
             if (GRAD) {
+                load_two(dRs + q * LR + ri, even, dR);
 #pragma unroll
                 for (int x = 0; x < 3; x++) dY[x] = dYs[(q * 3 + x) * L2 + lm];
             }
+            const double fY = D.f * Yv;
+            double g[3][2];
 #pragma unroll
             for (int j = 0; j < 2; j++) {
-                if (j == 1 && !has1) break;
-                const double Rv = Rs[q * LR + ri + j];
-                const double val = D.f * Yv * Rv;
+                const double val = fY * R[j];
                 acc[j] += D.inv ? sign_l * val : val;
                 if (!GRAD) continue;
-                const double dR = dRs[q * LR + ri + j];
-                double g[3];
+                const double fdR = D.f * dR[j], fR = D.f * R[j];
 #pragma unroll
-                for (int x = 0; x < 3; x++) g[x] = D.fg * D.u[x] * Rv * Yv + D.f * dR * D.u[x] * Yv + D.f * Rv * dY[x] * D.rinv;
-                const int k = lm * N + n0 + j;
-                if (POS && !D.inv) {
-                    double* pg = a.pair_grad + D.pair * 3 * K;
-                    pg[k] = g[0];
-                    pg[K + k] = g[1];
-                    pg[2 * K + k] = g[2];
-                }
-                const double gf = D.inv ? -sign_l : 1.0;
-                const double gi[3] = {gf * g[0], gf * g[1], gf * g[2]};
+                for (int x = 0; x < 3; x++) g[x][j] = D.fgu[x] * R[j] * Yv + fdR * D.u[x] * Yv + fR * dY[x] * D.rinv;
+            }
+            if (!GRAD) continue;
+            if (POS && !D.inv) {
+                double* pg = a.pair_grad + D.pair * 3 * K + k0;
+#pragma unroll
+                for (int x = 0; x < 3; x++) store_two(pg + x * K, even, has1, g[x]);
+            }
+            // times 1, or -(-1)^l for a reversed pair: exact
+            const bool negate = D.inv && !odd_l;
+#pragma unroll
+            for (int j = 0; j < 2; j++) {
+                double gi[3];
+#pragma unroll
+                for (int x = 0; x < 3; x++) gi[x] = negate ? -g[x][j] : g[x][j];
                 if (POS && !D.self_image) {
                     sg[j][0] -= gi[0];
                     sg[j][1] -= gi[1];
@@ -387,46 +475,41 @@ __global__ void __launch_bounds__(256, 2) se_fused_kernel(SeArgs a, DevicePairs 
                 }
                 if (STRAIN) {
 #pragma unroll
-                    for (int x = 0; x < 3; x++) {
-                        const double vx = D.inv ? -D.v[x] : D.v[x];
+                    for (int x = 0; x < 3; x++)
 #pragma unroll
-                        for (int y = 0; y < 3; y++) st[j][x * 3 + y] += vx * gi[y];
-                    }
+                        for (int y = 0; y < 3; y++) st[j][x * 3 + y] += D.v[x] * gi[y];
                 }
                 if (CELL) {
 #pragma unroll
-                    for (int x = 0; x < 3; x++) {
-                        const double sx = D.inv ? -D.sh[x] : D.sh[x];
+                    for (int x = 0; x < 3; x++)
 #pragma unroll
-                        for (int y = 0; y < 3; y++) ce[j][x * 3 + y] += sx * gi[y];
-                    }
+                        for (int y = 0; y < 3; y++) ce[j][x * 3 + y] += D.sh[x] * gi[y];
                 }
             }
         }
     }
     if (!active) return;
     const int64_t base = c * S + t;
+    const bool own = t == tc && l == 0;
+    const double self[2] = {own ? a.self_contribution[n0] : 0.0, own && has1 ? a.self_contribution[n0 + 1] : 0.0};
+    const double value[2] = {self[0] + acc[0], self[1] + acc[1]};
+    store_two(a.coef + base * K + k0, even, has1, value);
+    if (POS) {
 #pragma unroll
-    for (int j = 0; j < 2; j++) {
-        if (j == 1 && !has1) break;
-        const int n = n0 + j, k = lm * N + n;
-        const double self = (t == tc && l == 0) ? a.self_contribution[n] : 0.0;
-        a.coef[base * K + k] = self + acc[j];
-        if (POS) {
-            double* sgp = a.self_grad + base * 3 * K;
-            sgp[k] = sg[j][0];
-            sgp[K + k] = sg[j][1];
-            sgp[2 * K + k] = sg[j][2];
+        for (int x = 0; x < 3; x++) {
+            const double v[2] = {sg[0][x], sg[1][x]};
+            store_two(a.self_grad + (base * 3 + x) * K + k0, even, has1, v);
         }
-        if (STRAIN) {
-            double* o = a.strain + base * 9 * K;
+    }
 #pragma unroll
-            for (int x = 0; x < 9; x++) o[x * K + k] = st[j][x];
+    for (int x = 0; x < 9; x++) {
+        if (STRAIN) {
+            const double v[2] = {st[0][x], st[1][x]};
+            store_two(a.strain + (base * 9 + x) * K + k0, even, has1, v);
         }
         if (CELL) {
-            double* o = a.cellg + base * 9 * K;
-#pragma unroll
-            for (int x = 0; x < 9; x++) o[x * K + k] = ce[j][x];
+            const double v[2] = {ce[0][x], ce[1][x]};
+            store_two(a.cellg + (base * 9 + x) * K + k0, even, has1, v);
         }
     }
 }
@@ -580,7 +663,7 @@ void set_se_fused_enabled(bool enabled) { fused_state = enabled ? 1 : 0; }
 
 bool se_fused_supported(const FeatureLayout& layout, const DeviceRadial& radial, const DenseTables<double>& tables) {
     if (!layout.with_grad && centre_expansion_supported(tables)) return true;
-    const size_t bytes = sizeof(double) * fused_shared_doubles(layout.lmax, layout.nmax, layout.with_grad);
+    const size_t bytes = sizeof(double) * fused_shared_doubles(layout.lmax, layout.nmax, layout.with_grad, tables.spline.levels);
     const int items = layout.L2 * ((layout.nmax + 1) / 2);
     return radial.splined && layout.lmax <= LMAX_SMALL && items <= 256 && bytes <= 160 * 1024;
 }
@@ -609,7 +692,7 @@ void launch_se_fused(const SeArgs& args, const DevicePairs& pairs, const DeviceR
     const FeatureLayout& L = args.layout;
     const int items = L.L2 * ((L.nmax + 1) / 2);
     const int threads = std::max(32, (items + 31) / 32 * 32);
-    const size_t smem = sizeof(double) * fused_shared_doubles(L.lmax, L.nmax, L.with_grad);
+    const size_t smem = sizeof(double) * fused_shared_doubles(L.lmax, L.nmax, L.with_grad, tables.spline.levels);
     const bool grad = L.with_grad;
     const bool p = grad && args.do_positions, st = grad && args.do_strain, ce = grad && args.do_cell;
     const unsigned blocks = (unsigned)(args.n_centres * args.n_species);
@@ -617,7 +700,7 @@ void launch_se_fused(const SeArgs& args, const DevicePairs& pairs, const DeviceR
     do {                                                                                                              \
         CUDA_CHECK(cudaFuncSetAttribute(se_fused_kernel<P, ST, CE>, cudaFuncAttributeMaxDynamicSharedMemorySize,      \
                                         (int)smem));                                                                  \
-        se_fused_kernel<P, ST, CE><<<blocks, threads, smem, stream>>>(args, pairs, radial, ylm, cut);                 \
+        se_fused_kernel<P, ST, CE><<<blocks, threads, smem, stream>>>(args, pairs, radial, ylm, cut, tables.spline);                 \
     } while (0)
     if (!p && !st && !ce) SE_FUSED(false, false, false);
     else if (p && !st && !ce) SE_FUSED(true, false, false);
