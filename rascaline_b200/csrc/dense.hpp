@@ -130,6 +130,16 @@ void launch_dense_grad_coef_species(const DenseArgs<float>& a, cudaStream_t stre
 // tiles (species, first, count) over `order`, the atoms sorted by species
 std::vector<int32_t> dense_species_tiles(const std::vector<int32_t>& species, int n_species, std::vector<int32_t>& order);
 
+// tangent of the coefficients with one CTA per centre (dense_tangent.cu)
+template <typename T>
+void launch_dense_tangent_by_centre(const DenseArgs<T>& a, const T* tpos, const T* tcell, T* tcoef, cudaStream_t stream);
+// tangent of the power spectrum with a warp per centre (nmax <= 8, at most
+// four species, 2-value alignment of tvalues)
+template <typename T>
+bool dense_tangent_by_warp(const DenseArgs<T>& a, const T* tvalues);
+template <typename T>
+void launch_dense_tangent_warp(const DenseArgs<T>& a, const T* tcoef, T* tvalues, cudaStream_t stream);
+
 // What a batch of systems adds to a forward and backward pass of a linear
 // model: one row of weights per species
 struct SpeciesModel {

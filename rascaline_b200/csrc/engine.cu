@@ -1197,8 +1197,15 @@ void Engine::jvp_dense(DenseState& st, const void* tangent_positions, const void
     const size_t T_size = st.precision == 64 ? 8 : 4;
     const int64_t P = st.n_pairs;
     const FeatureLayout layout = FeatureLayout::make(h_.max_angular, h_.nmax(), true);
-    void* features = arena_.alloc_bytes("dense.features_grad", T_size * (size_t)std::max<int64_t>(P, 1) * layout.stride);
-    void* pair_tangent = arena_.alloc_bytes("dense.pair_tangent", T_size * (size_t)std::max<int64_t>(P, 1) * st.K);
+    // the tangent by centre needs no pair records
+    const bool records = st.precision == 32 ? active_surrogate_ != nullptr || !centre_expansion_supported(dense_f_)
+                                            : !centre_expansion_supported(dense_d_);
+    void* features = nullptr;
+    void* pair_tangent = nullptr;
+    if (records) {
+        features = arena_.alloc_bytes("dense.features_grad", T_size * (size_t)std::max<int64_t>(P, 1) * layout.stride);
+        pair_tangent = arena_.alloc_bytes("dense.pair_tangent", T_size * (size_t)std::max<int64_t>(P, 1) * st.K);
+    }
     void* tcoef = tangent_coef ? tangent_coef
                                : arena_.alloc_bytes("dense.tangent_coef", T_size * (size_t)st.n_atoms * st.n_species * st.K);
     int32_t* status = arena_.alloc<int32_t>("dense.status", 1);
