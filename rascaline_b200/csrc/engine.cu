@@ -837,7 +837,7 @@ std::unique_ptr<TensorMap> Engine::compute(int kind, std::vector<HostSystem>& sy
             pa.entry_offset = nb.entry_offset;
             pa.entries = nb.entries;
             pa.entry_cum = nb.entry_cum;
-            pa.slot_row = upload(arena_, "ps.slot_row", plan.slot_row, up);
+            if (g.positions) pa.slot_row = upload(arena_, "ps.slot_row", plan.slot_row, up);
             pa.off_values = upload(arena_, "ps.offv", offv, up);
             pa.off_positions = upload(arena_, "ps.offp", offp, up);
             pa.off_strain = upload(arena_, "ps.offs", offs, up);

@@ -250,8 +250,20 @@ OutputPlan plan_power_spectrum(const Neighborhoods& nh, const Hypers& h, const G
     }
     plan.blocks.resize(nb);
 
-    // slots, sample rows and the first gradient row of every slot
+    // slots, sample rows and (for positions) the first gradient row of every
+    // slot; the storage is sized at once (165 000 slots of molecules, grown by
+    // push_back with gradient rows nothing read, were the longest part of a
+    // call for values alone: 1.6 to 2.1 ms before the launch, now 1.06)
     plan.slot_offset.assign(N + 1, 0);
+    int64_t n_slots = 0;
+    for (int64_t c = 0; c < N; c++) {
+        const uint8_t* mask = &nh.species_mask[(size_t)c * S];
+        int64_t present = 0;
+        for (int a = 0; a < S; a++) present += mask[a] != 0;
+        n_slots += present * (present + 1) / 2;
+    }
+    plan.slots.reserve(n_slots);
+    if (g.positions) plan.slot_row.reserve(n_slots);
     for (int64_t c = 0; c < N; c++) {
         const uint8_t* mask = &nh.species_mask[(size_t)c * S];
         const int32_t* count = &nh.species_count[(size_t)c * S];
@@ -262,6 +274,7 @@ OutputPlan plan_power_spectrum(const Neighborhoods& nh, const Hypers& h, const G
                 int32_t k = key_index[((size_t)nh.atom_species[c] * S + a) * S + b];
                 auto& bp = plan.blocks[k];
                 plan.slots.push_back(PsKeySlot{k, (int32_t)bp.n_samples++, a, b});
+                if (!g.positions) continue;
                 plan.slot_row.push_back(bp.n_grad_rows);
                 bp.n_grad_rows += count[a] + (a != b ? count[b] : 0) + 1;
             }
