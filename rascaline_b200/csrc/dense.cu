@@ -6,18 +6,25 @@
 //                keeps pair order inside each segment, the order of
 //                featomic's accumulate_all_pairs (spherical_expansion.rs:
 //                101-358); segment starts by binary search
-//   features     thread per pair: cutoff, Y_lm, R_nl in T
-//   expansion    CTA per (centre, species), thread per (l, m, n), segment reduced in
-//                registers (no atomics), inverse pairs with (-1)^l
-//                (spherical_expansion_pair.rs:130-163), self term on l = 0
-//   contraction  CTA per centre, coefficients in shared memory, thread per
-//                (species pair a <= b, l, n1) with a register row over n2:
+//   expansion    CTA per centre, nothing stored per pair (centre_expansion.cuh);
+//                with a surrogate, an analytic radial integral or larger
+//                bases: a record per pair (thread per pair: cutoff, Y_lm, R_nl
+//                in T), then a CTA per (centre, species), thread per
+//                (l, m, n), segment reduced in registers (no atomics), inverse
+//                pairs with (-1)^l (spherical_expansion_pair.rs:130-163), self
+//                term on l = 0
+//   contraction  warp per centre on the tensor cores (dense_warp.cu); here, for
+//                the CUDA-core engine and larger bases: CTA per centre,
+//                coefficients in shared memory, thread per (species pair
+//                a <= b, l, n1) with a register row over n2:
 //                P[l n1 n2] = sum_m c_a[l m n1] c_b[l m n2] / ((-1)^l sqrt(2l+1)),
 //                times sqrt(2) when a != b (power_spectrum.rs:529-780)
 //
 // Backward (adjoint of the above for a loss L with dL/dP given):
-//   dL/dc        CTA per centre, coefficients and dL/dP in shared memory,
-//                thread per (a, l, n) with a register row over m:
+//   dL/dc        FP32 on tcgen05 (dense_mma.cu) or, with a row of weights per
+//                species, and in FP64, a warp per centre or tile of centres
+//                (dense_warp.cu); here CTA per centre, coefficients and dL/dP in
+//                shared memory, thread per (a, l, n) with a register row over m:
 //                dL/dc_a[l m n] = sum over the species pairs containing a of
 //                scale * sum_n' G[n n'] c_b[l m n']
 //   dL/dr_ij     thread per pair, Y_lm, dY_lm, R_nl, dR_nl recomputed in
