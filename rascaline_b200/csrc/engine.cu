@@ -305,7 +305,17 @@ Engine::Engine(const Hypers& h) : h_(h) {
 }
 
 Engine::~Engine() {
-    for (void* p : table_buffers_) cudaFree(p);
+    if (!table_buffers_.empty()) {
+        // The tables are pool memory, which cudaFree gives back without
+        // waiting (for cudaMalloc's memory it waits by itself), and the dense
+        // forms return with kernels queued that read them
+        int current = device_;
+        cudaGetDevice(&current);
+        if (current != device_) cudaSetDevice(device_);
+        cudaDeviceSynchronize();
+        for (void* p : table_buffers_) cudaFree(p);
+        if (current != device_) cudaSetDevice(current);
+    }
     if (staging_) cudaFreeHost(staging_);
     if (dense_marks_ready_)
         for (auto& e : dense_marks_) cudaEventDestroy(e);
