@@ -333,6 +333,7 @@ __global__ void __launch_bounds__(32 * PV_WARPS, 3) ps_values_tiles_kernel(PsArg
         rows[slot.a * NS - slot.a * (slot.a - 1) / 2 + slot.b - slot.a] = out;
         aligned = aligned && ((uintptr_t)out & 15) == 0;
     }
+    __syncwarp();  // the rows above are read by every lane; the vote orders no memory
     aligned = __all_sync(0xffffffffu, aligned);
     const bool row = g < N, lower = row && 2 * t < N, upper = row && 2 * t + 1 < N;
     const double* X = a.coef + c * NS * (int64_t)K + N * t + (row ? g : 0);

@@ -45,3 +45,29 @@ def test_values(atoms, species, max_radial, max_angular):
         np.testing.assert_allclose(block.values, expected, rtol=0.0, atol=1e-12 * np.abs(dense).max())
         seen[rows, pair] = True
     np.testing.assert_array_equal(dense[~seen], 0.0)
+
+
+def test_every_slot_of_many_centres():
+    """Rows of one to ten slots a centre, thousands of warps in flight: no part
+    of a tile is dropped, and repeated calls agree to the last bit."""
+    systems = workloads.molecules(256, seed=3)
+    sizes = [len(m["types"]) for m in systems]
+    types = np.concatenate([m["types"] for m in systems])
+    positions = np.concatenate([m["positions"] for m in systems])
+    calculator = rb.SoapPowerSpectrum(**workloads.hypers(3.0, 7, 3))
+    dense, _ = torch_api.dense_power_spectrum(calculator, torch.tensor(positions, device="cuda"), types,
+                                              np.zeros((len(sizes), 9)), sizes, 64)
+    dense = dense.cpu().numpy()
+    start = np.concatenate([[0], np.cumsum(sizes)])
+    present = sorted(set(types.tolist()))
+    pairs = [(a, b) for i, a in enumerate(present) for b in present[i:]]
+    first = None
+    for _ in range(3):
+        result = calculator.compute(systems)
+        found = np.zeros_like(dense)
+        for key, block in zip(result.keys.values.tolist(), result.blocks()):
+            samples = np.asarray(block.samples.values)
+            found[start[samples[:, 0]] + samples[:, 1], pairs.index((key[1], key[2]))] = np.asarray(block.values)
+        np.testing.assert_allclose(found, dense, rtol=0.0, atol=1e-12 * np.abs(dense).max())
+        first = found if first is None else first
+        np.testing.assert_array_equal(found, first)
