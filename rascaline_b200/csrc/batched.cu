@@ -120,6 +120,7 @@ BatchPlan::BatchPlan(Engine& engine, const std::vector<int64_t>& sizes, const st
     d_atom_energy_ = (float*)put(nullptr, sizeof(float) * (size_t)std::max<int64_t>(n_atoms_, 1));
     d_atom_strain_ = (float*)put(nullptr, sizeof(float) * 9 * (size_t)std::max<int64_t>(n_atoms_, 1));
     CUDA_CHECK(cudaMemset(d_control_, 0, 64));
+    finish_copies();
     CUDA_CHECK(cudaStreamCreateWithFlags(&capture_stream_, cudaStreamNonBlocking));
     systems_.resize(sizes.size());
     for (size_t s = 0; s < sizes.size(); s++) {

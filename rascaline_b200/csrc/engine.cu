@@ -368,7 +368,7 @@ void Engine::upload_tables() {
     const size_t room = ((size_t)1 << 18) + sizeof(double) * (radial_.positions.size() * 4 + radial_.values.size() * 16 +
                                                              radial_.ortho.size() * 4);
     // (from the pool: cudaMalloc maps new memory for a block of this size, 2 ms
-    // of the first call of every calculator; the copy below waits for both)
+    // of the first call of every calculator)
     unsigned char* base = nullptr;
     CUDA_CHECK(cudaMallocAsync((void**)&base, room, cudaStreamLegacy));
     table_buffers_.push_back(base);
@@ -503,6 +503,7 @@ void Engine::upload_tables() {
     }
     dense_f_.self_contribution = putf(radial_.self_contribution);
     CUDA_CHECK(cudaMemcpy(base, staged.data(), staged.size(), cudaMemcpyHostToDevice));
+    finish_copies();
     tables_ready_ = true;
 }
 

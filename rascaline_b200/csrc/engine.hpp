@@ -23,6 +23,12 @@
 
 namespace fb200 {
 
+// cudaMemcpy from pageable memory returns when the source is staged, with the
+// transfer itself still to come, and the engine's streams (and a caller's
+// non-blocking one) are not ordered after it: waits until what was copied or
+// set so far is in device memory
+inline void finish_copies() { CUDA_CHECK(cudaStreamSynchronize(cudaStreamLegacy)); }
+
 // Named, growing device buffers reused across calls of one calculator.
 class DeviceArena {
   public:

@@ -786,6 +786,7 @@ void LodeEngine::upload_tables() {
     CUDA_CHECK(cudaMalloc(&d, pack.bytes.size()));
     table_buffers_.push_back(d);
     CUDA_CHECK(cudaMemcpy(d, pack.bytes.data(), pack.bytes.size(), cudaMemcpyHostToDevice));
+    finish_copies();
     auto dbl = [&](int k) { return reinterpret_cast<const double*>(d + at[k]); };
     d_ylm_ = {ylm_.lmax, dbl(0), dbl(1), dbl(2), dbl(3), dbl(4), dbl(5), dbl(6), dbl(7)};
     d_spline_.lmax = tables_.h.max_angular;

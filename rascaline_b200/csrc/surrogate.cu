@@ -579,6 +579,7 @@ RadialSurrogate::RadialSurrogate(Engine& engine, int hidden, uint64_t seed) : en
     CUDA_CHECK(cudaMemset(d_step_, 0, 8));
     scale_.assign(O_, 1.0f);
     CUDA_CHECK(cudaMemcpy(d_scale_, scale_.data(), 4 * O_, cudaMemcpyHostToDevice));
+    finish_copies();
 }
 
 RadialSurrogate::~RadialSurrogate() {
