@@ -262,7 +262,7 @@ BatchPlan::Shape BatchPlan::shape(const BatchArgs& a, const BatchConfig& c) cons
     sh.smem = shared_bytes(a, c);
     sh.threads = 32 * c.warps;
     if (sh.smem > 227 * 1024) return sh;
-    CUDA_CHECK(cudaFuncSetAttribute((const void*)sh.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem));
+    allow_shared_memory((const void*)sh.fn, sh.smem);
     int per_sm = 0;
     CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)sh.fn, sh.threads, sh.smem));
     int sms = 0;

@@ -333,8 +333,7 @@ void launch_centre_expansion(const CentreArgs<T>& a, cudaStream_t stream) {
     if (a.n_centres == 0) return;
     const CentreLayout<T> lay(a.ylm.lmax, a.spline.nmax, a.spline.levels);
     auto run = [&](auto kernel) {
-        if (lay.bytes > 48 * 1024)
-            CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lay.bytes));
+        allow_shared_memory(kernel, lay.bytes);
         kernel<<<(unsigned)a.n_centres, CE_THREADS, lay.bytes, stream>>>(a);
     };
     if (a.spline.nmax <= 8) run(centre_expansion_kernel<T, 8>);

@@ -580,8 +580,7 @@ bool cg_product_mma(const featomic_b200_cg_task_t* tasks, size_t n_tasks, cudaSt
     CUDA_CHECK(cudaMallocAsync(reinterpret_cast<void**>(&buffer), host.size(), stream));
     // staged before the call returns (pageable source)
     CUDA_CHECK(cudaMemcpyAsync(buffer, host.data(), host.size(), cudaMemcpyHostToDevice, stream));
-    CUDA_CHECK(cudaFuncSetAttribute(cg_product_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)std::max<size_t>(smem, 48 * 1024)));
+    allow_shared_memory(cg_product_mma_kernel, smem);
     cg_product_mma_kernel<<<(unsigned)blocks, 32 * CG_MMA_WARPS, smem, stream>>>(
         reinterpret_cast<const DeviceCgGroup*>(buffer), (int)groups.size(), reinterpret_cast<const CgRow*>(buffer + gb),
         reinterpret_cast<const CgCoef*>(buffer + gb + rb), (int)warp_doubles);

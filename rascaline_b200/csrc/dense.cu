@@ -918,14 +918,6 @@ template <typename T>
 void launch_dense_grad_coef(const DenseArgs<T>& a, cudaStream_t stream) {
     const size_t smem = sizeof(T) * (size_t)a.n_species * a.K;
     if (smem > 200 * 1024) throw invalid_parameter("too many species x coefficients for the adjoint kernel");
-    static bool configured[2] = {false, false};
-    const int which = sizeof(T) == 8 ? 1 : 0;
-    if (!configured[which]) {
-        CUDA_CHECK(cudaFuncSetAttribute(dense_grad_coef<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-        CUDA_CHECK(cudaFuncSetAttribute(dense_grad_coef_tiled<T, 17>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        200 * 1024));
-        configured[which] = true;
-    }
     const size_t tiled_smem = smem + sizeof(T) * (size_t)a.n_keys * a.n_props;
     bool mma = false;
     if constexpr (sizeof(T) == 4) mma = dense_mma_enabled() && dense_mma_supported(a);
@@ -942,8 +934,10 @@ void launch_dense_grad_coef(const DenseArgs<T>& a, cudaStream_t stream) {
     } else if (mma) {
         if constexpr (sizeof(T) == 4) launch_dense_grad_coef_mma(a, stream);
     } else if (a.lmax <= DENSE_LMAX_SMALL && tiled_smem <= 200 * 1024) {
+        allow_shared_memory(dense_grad_coef_tiled<T, 17>, tiled_smem);
         dense_grad_coef_tiled<T, 17><<<(unsigned)a.n_atoms, 128, tiled_smem, stream>>>(a);
     } else {
+        allow_shared_memory(dense_grad_coef<T>, smem);
         dense_grad_coef<T><<<(unsigned)a.n_atoms, 256, smem, stream>>>(a);
     }
     CUDA_CHECK(cudaGetLastError());

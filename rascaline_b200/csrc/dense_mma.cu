@@ -317,7 +317,7 @@ void launch_persistent(Kernel kernel, const DenseArgs<float>& a, const MmaShape&
                        cudaStream_t stream) {
     const int max_ctas = std::min(4, 512 / sh.tmem_cols);
     const size_t request = std::max<size_t>(smem + 1024, 228 * 1024 / (max_ctas + 1) + 1024);
-    CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)request));
+    allow_shared_memory(kernel, request);
     CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                     (int)cudaSharedmemCarveoutMaxShared));
     // resident CTAs per SM from the shared-memory request (228 KB per SM,

@@ -227,8 +227,7 @@ template <typename T>
 void launch_dense_tangent_by_centre(const DenseArgs<T>& a, const T* tpos, const T* tcell, T* tcoef, cudaStream_t stream) {
     const TangentLayout<T> lay(a.lmax, a.nmax, a.tab.spline.levels);
     auto run = [&](auto kernel) {
-        if (lay.bytes > 48 * 1024)
-            CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lay.bytes));
+        allow_shared_memory(kernel, lay.bytes);
         kernel<<<(unsigned)a.n_atoms, CE_THREADS, lay.bytes, stream>>>(a, tpos, tcell, tcoef);
     };
     if (a.nmax <= 8) run(centre_tangent_kernel<T, 8>);

@@ -278,6 +278,24 @@ void join_uploads(cudaStream_t stream) {
     CUDA_CHECK(cudaEventDestroy(done));  // released once the recorded work has completed
 }
 
+}  // namespace
+
+void allow_shared_memory(const void* kernel, size_t bytes) {
+    static std::mutex mutex;
+    static std::map<std::pair<int, const void*>, size_t> limits;
+    int device = 0;
+    CUDA_CHECK(cudaGetDevice(&device));
+    std::lock_guard<std::mutex> lock(mutex);
+    size_t& limit = limits[{device, kernel}];
+    if (bytes <= limit) return;
+    // 48 KB of dynamic memory beside any static memory are within the device's limit
+    const size_t request = std::max<size_t>(bytes, 48 * 1024);
+    CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)request));
+    limit = request;
+}
+
+namespace {
+
 double elapsed_ms(cudaEvent_t a, cudaEvent_t b) {
     float ms = 0.0f;
     if (cudaEventElapsedTime(&ms, a, b) != cudaSuccess) {

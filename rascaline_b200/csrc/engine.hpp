@@ -29,6 +29,15 @@ namespace fb200 {
 // set so far is in device memory
 inline void finish_copies() { CUDA_CHECK(cudaStreamSynchronize(cudaStreamLegacy)); }
 
+// Raises a kernel's limit on dynamic shared memory to at least `bytes`, for a
+// launch that follows.  The limit is the process's, per device: it is never
+// lowered, since another thread may be about to launch the same kernel with more.
+void allow_shared_memory(const void* kernel, size_t bytes);
+template <typename... Args>
+void allow_shared_memory(void (*kernel)(Args...), size_t bytes) {
+    allow_shared_memory(reinterpret_cast<const void*>(kernel), bytes);
+}
+
 // Named, growing device buffers reused across calls of one calculator.
 class DeviceArena {
   public:

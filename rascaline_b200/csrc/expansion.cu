@@ -698,9 +698,8 @@ void launch_se_fused(const SeArgs& args, const DevicePairs& pairs, const DeviceR
     const unsigned blocks = (unsigned)(args.n_centres * args.n_species);
 #define SE_FUSED(P, ST, CE)                                                                                           \
     do {                                                                                                              \
-        CUDA_CHECK(cudaFuncSetAttribute(se_fused_kernel<P, ST, CE>, cudaFuncAttributeMaxDynamicSharedMemorySize,      \
-                                        (int)smem));                                                                  \
-        se_fused_kernel<P, ST, CE><<<blocks, threads, smem, stream>>>(args, pairs, radial, ylm, cut, tables.spline);                 \
+        allow_shared_memory(se_fused_kernel<P, ST, CE>, smem);                                                        \
+        se_fused_kernel<P, ST, CE><<<blocks, threads, smem, stream>>>(args, pairs, radial, ylm, cut, tables.spline);  \
     } while (0)
     if (!p && !st && !ce) SE_FUSED(false, false, false);
     else if (p && !st && !ce) SE_FUSED(true, false, false);
@@ -842,8 +841,7 @@ void launch_se_output(const SeOutArgs& args, bool positions, bool strain, bool c
     CUDA_CHECK(cudaGetLastError());
     if (positions) {
         const size_t smem = sizeof(int) * (size_t)(args.lmax + 1) * (args.lmax + 1) * args.nmax;
-        if (smem > 48 * 1024)
-            CUDA_CHECK(cudaFuncSetAttribute(se_output_gradients_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        allow_shared_memory(se_output_gradients_kernel, smem);
         se_output_gradients_kernel<<<(unsigned)(args.n_centres * SE_SPLIT), 256, smem, stream>>>(args);
         CUDA_CHECK(cudaGetLastError());
     }

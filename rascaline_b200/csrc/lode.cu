@@ -1012,6 +1012,7 @@ std::unique_ptr<TensorMap> LodeEngine::compute(const std::vector<HostSystem>& sy
         // k-vectors per CTA of the projection: at most 8 and 48 KB of shared memory
         const size_t per_k = sizeof(double) * (size_t)((L + 1) * (L + 2) / 2 + L2 + (L + 1) * N);
         const int kc = (int)std::max<size_t>(1, std::min<size_t>(8, 48 * 1024 / per_k));
+        allow_shared_memory(lode_projection_kernel, kc * per_k);
         lode_projection_kernel<<<(Kp + kc - 1) / kc, 128, kc * per_k, stream>>>(
             K, Kp, kc, N, a.cols, doubles(o_dir), doubles(o_norm), h.splined ? nullptr : doubles(o_radial), d_spline_, d_ylm_,
             T);

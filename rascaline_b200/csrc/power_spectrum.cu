@@ -1148,16 +1148,6 @@ void launch_all(const PsArgs& args, bool values, bool positions, bool strain, bo
     const int K = (args.lmax + 1) * (args.lmax + 1) * args.nmax;
     const size_t coef_bytes = sizeof(double) * ((size_t)args.n_species * K + 2 * (args.lmax + 1));
     const int threads = 256;
-    static bool configured = false;
-    if (!configured) {
-        CUDA_CHECK(cudaFuncSetAttribute(ps_values_kernel<MAXN>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-        CUDA_CHECK(cudaFuncSetAttribute(ps_positions_kernel<MAXN>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-        CUDA_CHECK(cudaFuncSetAttribute(ps_strain_cell_kernel<MAXN>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-        CUDA_CHECK(cudaFuncSetAttribute(ps_positions_staged_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-        CUDA_CHECK(cudaFuncSetAttribute(ps_positions_staged_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-        CUDA_CHECK(cudaFuncSetAttribute(ps_centre_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-        configured = true;
-    }
     if (coef_bytes > 200 * 1024) throw invalid_parameter("too many species / radial / angular functions for the power spectrum kernels");
     const size_t pos_bytes =
         sizeof(double) * (((size_t)args.n_species * K + 2 * (args.lmax + 1) + 1) / 2 * 2) + POS_TABLE_BYTES;
@@ -1191,15 +1181,18 @@ void launch_all(const PsArgs& args, bool values, bool positions, bool strain, bo
         else ps_values_tiles_kernel<4><<<grid, 32 * PV_WARPS, 0, side>>>(args);
         CUDA_CHECK(cudaGetLastError());
     } else if (values && !centre_rows) {
+        allow_shared_memory(ps_values_kernel<MAXN>, coef_bytes);
         ps_values_kernel<MAXN><<<(unsigned)args.n_centres, threads, coef_bytes, side>>>(args);
         CUDA_CHECK(cudaGetLastError());
     }
     if (events.after_values) CUDA_CHECK(cudaEventRecord(events.after_values, side));
     if (centre_rows) {
+        allow_shared_memory(ps_centre_rows_kernel, cr_bytes);
         ps_centre_rows_kernel<<<(unsigned)(CR_SPLIT * args.n_centres), 128, cr_bytes, side>>>(args, kinds);
         CUDA_CHECK(cudaGetLastError());
     } else {
         if (staged) throw std::logic_error("the centres' own rows need ps_centre_rows_kernel");
+        allow_shared_memory(ps_strain_cell_kernel<MAXN>, coef_bytes);
         if (strain) {
             ps_strain_cell_kernel<MAXN><<<(unsigned)args.n_centres, threads, coef_bytes, side>>>(args, 0);
             CUDA_CHECK(cudaGetLastError());
@@ -1217,9 +1210,12 @@ void launch_all(const PsArgs& args, bool values, bool positions, bool strain, bo
     if (positions) {
         if (staged) {
             const unsigned grid = (unsigned)(args.n_centres * STG_SPLIT);
+            allow_shared_memory(ps_positions_staged_kernel<true>, stg.bytes);
+            allow_shared_memory(ps_positions_staged_kernel<false>, stg.bytes);
             if (args.nmax == 8) ps_positions_staged_kernel<true><<<grid, STG_WARPS * 32, stg.bytes, stream>>>(args);
             else ps_positions_staged_kernel<false><<<grid, STG_WARPS * 32, stg.bytes, stream>>>(args);
         } else {
+            allow_shared_memory(ps_positions_kernel<MAXN>, pos_bytes);
             ps_positions_kernel<MAXN><<<(unsigned)(args.n_centres * POS_SPLIT), POS_WARPS * 32, pos_bytes, stream>>>(args);
         }
         CUDA_CHECK(cudaGetLastError());

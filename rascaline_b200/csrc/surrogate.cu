@@ -848,7 +848,7 @@ void RadialSurrogate::fit_output_layer(double lambda, cudaStream_t stream) {
         CUDA_CHECK(cudaGetLastError());
     }
     const size_t smem = sizeof(double) * (size_t)F * W;
-    CUDA_CHECK(cudaFuncSetAttribute(surrogate_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_shared_memory(surrogate_solve_kernel, smem);
     surrogate_solve_kernel<<<1, 256, smem, stream>>>(M, O_, d_master_, status);
     CUDA_CHECK(cudaGetLastError());
     int32_t h_status = 0;

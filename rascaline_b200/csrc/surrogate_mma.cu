@@ -345,8 +345,7 @@ void launch_surrogate_mma(const float* master, int hidden, int O, int out_pad, d
     // request keeps a third off any SM)
     const size_t smem_request = std::max<size_t>(smem, 228 * 1024 / 3 + 1024);
     if (smem_request > 227 * 1024) throw invalid_parameter("the tensor-core surrogate kernel supports at most 128 outputs");
-    CUDA_CHECK(cudaFuncSetAttribute(surrogate_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)smem_request));
+    allow_shared_memory(surrogate_mma_kernel, smem_request);
     // the largest shared-memory carveout
     CUDA_CHECK(cudaFuncSetAttribute(surrogate_mma_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                     (int)cudaSharedmemCarveoutMaxShared));
