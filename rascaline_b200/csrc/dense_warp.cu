@@ -127,43 +127,15 @@ __device__ __forceinline__ void step_upper(double (&acc)[NT + 1][NT][2], const d
         for (int j = i; j < NT; j++) mma_f64(acc[i][j], x[i][0], x[j][0]);
 }
 
-// ... and of D^T X + X^T D; the error against 64 bits is that of FP32 FMAs
-// (1.45e-6 of the norm for both at 6000 atoms: it is the coefficients')
+// ... and of four m of D^T X + X^T D
 template <int NT>
-__device__ __forceinline__ void step_upper2(float (&acc)[NT + 1][NT][2], const float (&x)[NT][2], const float (&d)[NT][2]) {
-    uint32_t h[2][NT + 1][2], l[2][NT + 1][2];
-#pragma unroll
-    for (int e = 0; e < 2; e++) {
-        h[0][NT][e] = l[0][NT][e] = h[1][NT][e] = l[1][NT][e] = 0;
-#pragma unroll
-        for (int j = 0; j < NT; j++) {
-            split(x[j][e], h[0][j][e], l[0][j][e]);
-            split(d[j][e], h[1][j][e], l[1][j][e]);
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < NT; i += 2)
-#pragma unroll
-        for (int j = i; j < NT; j++)
-#pragma unroll
-            for (int s = 0; s < 2; s++) {
-                const uint32_t(&ah)[NT + 1][2] = h[s];
-                const uint32_t(&al)[NT + 1][2] = l[s];
-                const uint32_t(&bh)[NT + 1][2] = h[1 - s];
-                const uint32_t(&bl)[NT + 1][2] = l[1 - s];
-                mma_tf32(acc[i][j], acc[i + 1][j], ah[i][0], ah[i + 1][0], ah[i][1], ah[i + 1][1], bh[j][0], bh[j][1]);
-                mma_tf32(acc[i][j], acc[i + 1][j], ah[i][0], ah[i + 1][0], ah[i][1], ah[i + 1][1], bl[j][0], bl[j][1]);
-                mma_tf32(acc[i][j], acc[i + 1][j], al[i][0], al[i + 1][0], al[i][1], al[i + 1][1], bh[j][0], bh[j][1]);
-            }
-}
-template <int NT>
-__device__ __forceinline__ void step_upper2(double (&acc)[NT + 1][NT][2], const double (&x)[NT][1], const double (&d)[NT][1]) {
+__device__ __forceinline__ void step_upper2(double (&acc)[NT][NT][2], const double (&x)[NT], const double (&d)[NT]) {
 #pragma unroll
     for (int i = 0; i < NT; i++)
 #pragma unroll
         for (int j = i; j < NT; j++) {
-            mma_f64(acc[i][j], x[i][0], d[j][0]);
-            mma_f64(acc[i][j], d[i][0], x[j][0]);
+            mma_f64(acc[i][j], x[i], d[j]);
+            mma_f64(acc[i][j], d[i], x[j]);
         }
 }
 
@@ -246,14 +218,16 @@ dense_contraction_tiles(DenseArgs<T> a, const T* __restrict__ weights, T* __rest
 
 // Tangent of the power spectrum, dP = dX^T X + X^T dX, by the same tiles: a
 // warp per centre (the CUDA-core kernel with a warp per species pair reads
-// four coefficients for two multiply-adds).  Bound by its stores and the load
-// latency of a warp's serial steps.  1500 atoms, 3 species, lmax 6, nmax 8,
-// FP32: 12 us (57 on the CUDA cores).
+// four coefficients for two multiply-adds).  FP32 coefficients are multiplied
+// and summed in FP64 as well: TF32 operands split into hi + lo, as for the
+// values, are four times as far from the exact products as the CUDA cores'
+// FP32 multiply-adds (2.1e-7 against 5.3e-8 of the norm).  Bound by its stores
+// and the load latency of a warp's serial steps.  1500 atoms, 3 species,
+// lmax 6, nmax 8, FP32: 13 us (57 on the CUDA cores, 12 with TF32).
 template <typename T, int NT, bool N8>
 __global__ void __launch_bounds__(32 * DW_WARPS, 2)
 dense_tangent_tiles(DenseArgs<T> a, const T* __restrict__ tcoef, T* __restrict__ tvalues) {
-    constexpr int E = sizeof(T) == 4 ? 2 : 1, STEP = 4 * E;
-    __shared__ T scales[64];
+    __shared__ double scales[64];
     fill_scales(scales);
     __syncthreads();
     const int lane = threadIdx.x & 31, t = lane & 3, g = lane >> 2;
@@ -266,34 +240,31 @@ dense_tangent_tiles(DenseArgs<T> a, const T* __restrict__ tcoef, T* __restrict__
 #pragma unroll 1
     for (int l = 0; l <= a.lmax; l++) {
         const int M = 2 * l + 1;
-        T acc[NT + 1][NT][2];
+        double acc[NT][NT][2];
 #pragma unroll
-        for (int i = 0; i <= NT; i++)
+        for (int i = 0; i < NT; i++)
 #pragma unroll
-            for (int j = 0; j < NT; j++) acc[i][j][0] = acc[i][j][1] = T(0);
+            for (int j = 0; j < NT; j++) acc[i][j][0] = acc[i][j][1] = 0.0;
 #pragma unroll 1
-        for (int m0 = 0; m0 < M; m0 += STEP) {
-            T x[NT][E], d[NT][E];
+        for (int m0 = 0; m0 < M; m0 += 4) {
+            double x[NT], d[NT];
+            const bool ok = m0 + t < M && row;
 #pragma unroll
-            for (int e = 0; e < E; e++) {
-                const bool ok = m0 + t + 4 * e < M && row;
-#pragma unroll
-                for (int i = 0; i < NT; i++) {
-                    x[i][e] = ok ? __ldg(a.coef + at + i * K + N * (m0 + 4 * e)) : T(0);
-                    d[i][e] = ok ? __ldg(tcoef + at + i * K + N * (m0 + 4 * e)) : T(0);
-                }
+            for (int i = 0; i < NT; i++) {
+                x[i] = ok ? (double)__ldg(a.coef + at + i * K + N * m0) : 0.0;
+                d[i] = ok ? (double)__ldg(tcoef + at + i * K + N * m0) : 0.0;
             }
             step_upper2<NT>(acc, x, d);
         }
         at += N * M;
-        const T same = scales[l], other = scales[32 + l];
+        const double same = scales[l], other = scales[32 + l];
         int key = 0;
 #pragma unroll
         for (int i = 0; i < NT; i++)
 #pragma unroll
             for (int j = i; j < NT; j++, key++) {
-                const T scale = i != j ? other : same;
-                const T v0 = acc[i][j][0] * scale, v1 = acc[i][j][1] * scale;
+                const double scale = i != j ? other : same;
+                const T v0 = (T)(acc[i][j][0] * scale), v1 = (T)(acc[i][j][1] * scale);
                 if (two) {
                     store2(out + key * P, v0, v1);
                 } else if (one) {

@@ -75,3 +75,37 @@ def test_tangent(species, max_radial, max_angular):
     fast, exact, cores = results[32, 1], results[64, 1], results[32, 0]
     assert float((fast - exact).abs().max()) <= 2e-5 * float(exact.abs().max())
     assert float((fast - cores).abs().max()) <= 2e-6 * float(exact.abs().max())
+
+
+@pytest.mark.parametrize("species,max_radial,max_angular", [(1, 0, 0), (2, 2, 3), (3, 7, 6), (4, 4, 5), (4, 7, 8)])
+def test_contraction_in_64_bits(species, max_radial, max_angular):
+    """The FP32 tangent of the power spectrum from its own FP32 coefficients and
+    their tangents: products and sums in 64 bits, one rounding at the end, so
+    |x - ref| <= 2^-24 |ref| + 2^-48 of the sum of sizes."""
+    systems = _systems(species)
+    hypers = workloads.hypers(3.6, max_radial, max_angular)
+    types = np.concatenate([s[0] for s in systems])
+    positions = torch.tensor(np.concatenate([s[1] for s in systems]), device="cuda")
+    cells = np.stack([s[2].reshape(9) for s in systems])
+    sizes = [len(s[0]) for s in systems]
+    move = torch.randn((len(types), 3), generator=torch.Generator().manual_seed(4)).cuda()
+    c, state = torch_api.dense_spherical_expansion(rb.SphericalExpansion(**hypers), positions, types, cells, sizes, 32)
+    state.expansion_width = c.shape[2]
+    _, d = torch_api.dense_jvp(state, move, values=False, coefficients=True)
+    _, state = torch_api.dense_power_spectrum(rb.SoapPowerSpectrum(**hypers), positions, types, cells, sizes, 32)
+    tangent, _ = torch_api.dense_jvp(state, move)
+    N, S = max_radial + 1, c.shape[1]
+    c, d = (x.double().reshape(len(types), S, (max_angular + 1) ** 2, N) for x in (c, d))
+    key = 0
+    for a in range(S):
+        for b in range(a, S):
+            for l in range(max_angular + 1):
+                x, y = (c[:, s, l * l:(l + 1) ** 2] for s in (a, b))
+                dx, dy = (d[:, s, l * l:(l + 1) ** 2] for s in (a, b))
+                scale = (-1) ** l / np.sqrt(2 * l + 1) * (np.sqrt(2) if a != b else 1)
+                product = lambda u, v: torch.einsum("cmp,cmq->cpq", u, v).reshape(len(types), -1)  # noqa: E731
+                reference = scale * (product(dx, y) + product(x, dy))
+                size = abs(scale) * (product(dx.abs(), y.abs()) + product(x.abs(), dy.abs()))
+                found = tangent[:, key, l * N * N:(l + 1) * N * N].double()
+                assert bool(((found - reference).abs() <= 2.0 ** -24 * reference.abs() + 2.0 ** -48 * size).all())
+            key += 1
