@@ -573,9 +573,14 @@ __global__ void __launch_bounds__(32 * DW_WARPS) dense_grad_coef_species(DenseAr
 
 template <typename T>
 bool dense_contraction_by_warp(const DenseArgs<T>& a) {
-    // FP32 as the CUDA cores' contraction where that is asked for; two values
-    // are stored at a time
-    return (sizeof(T) == 8 || dense_mma_enabled()) && a.lmax < 32 && (uintptr_t)a.values % (2 * sizeof(T)) == 0;
+    // two values are stored at a time
+    if (sizeof(T) == 8) return a.lmax < 32 && (uintptr_t)a.values % 16 == 0;
+    // FP32 as the CUDA cores' contraction where that is asked for, and where the
+    // tensor cores' dL/dc does not follow: FP32 multiply-adds are four times as
+    // close to the exact products as TF32 operands split into hi + lo (3.7e-8
+    // against 1.3e-7 of the norm)
+    if constexpr (sizeof(T) == 4) return dense_mma_enabled() && dense_mma_supported(a) && (uintptr_t)a.values % 16 == 0;
+    return false;
 }
 template bool dense_contraction_by_warp<float>(const DenseArgs<float>&);
 template bool dense_contraction_by_warp<double>(const DenseArgs<double>&);

@@ -106,3 +106,35 @@ def test_batch_weights_by_species(molecules, species, max_radial, max_angular):
     energies = torch.stack([x.sum() for x in torch.split(per_atom, sizes)])
     size = torch.stack([x.abs().sum() for x in torch.split(per_atom, sizes)])
     assert bool(((out["energies"] - energies).abs() <= 1e-5 * size).all())
+
+
+@pytest.mark.parametrize("atoms,species,max_radial,max_angular", [(40, 17, 7, 1), (30, 2, 3, 16), (24, 3, 2, 18)])
+def test_large_bases_keep_fp32_products(atoms, species, max_radial, max_angular):
+    """More than 128 (s, n) or l from 16 on: FP32 multiply-adds, as with the
+    tensor cores off, so that every value is within (M + 2) 2^-24 of the sum of
+    sizes of the products of its FP32 coefficients (M <= 2 l + 1 of them, and
+    the scale)."""
+    types = np.random.default_rng(atoms).permutation([1 + k % species for k in range(atoms)])
+    system = workloads.random_box(atoms, seed=atoms, species=(1,))
+    positions, cell = torch.tensor(system["positions"], device="cuda"), np.asarray(system["cell"]).reshape(1, 9)
+    hypers = workloads.hypers(3.5, max_radial, max_angular)
+    calculator = rb.SoapPowerSpectrum(**hypers)
+    results = []
+    for engine in (1, 0):
+        C.check(C.lib().featomic_b200_set_contraction_engine(engine, 1))
+        results.append(torch_api.dense_power_spectrum(calculator, positions, types, cell, [atoms], 32)[0])
+    assert torch.equal(*results)
+    c, _ = torch_api.dense_spherical_expansion(rb.SphericalExpansion(**hypers), positions, types, cell, [atoms], 32)
+    N = max_radial + 1
+    c = c.double().reshape(atoms, species, (max_angular + 1) ** 2, N)
+    key = 0
+    for a in range(species):
+        for b in range(a, species):
+            for l in range(max_angular + 1):
+                x, y = (c[:, s, l * l:(l + 1) ** 2] for s in (a, b))
+                scale = (-1) ** l / np.sqrt(2 * l + 1) * (np.sqrt(2) if a != b else 1)
+                reference = torch.einsum("cmp,cmq->cpq", x, y).reshape(atoms, -1) * scale
+                size = torch.einsum("cmp,cmq->cpq", x.abs(), y.abs()).reshape(atoms, -1) * abs(scale)
+                found = results[0][:, key, l * N * N:(l + 1) * N * N].double()
+                assert bool(((found - reference).abs() <= (2 * l + 3) * 2.0 ** -24 * size + 1e-40).all())
+            key += 1
