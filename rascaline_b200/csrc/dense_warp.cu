@@ -147,7 +147,9 @@ __device__ __forceinline__ void step_upper2(double (&acc)[NT][NT][2], const doub
 // (below) 0.174.  FP64, 2000 atoms: 17 us, 52 with a CTA per centre.
 // `energy`: with a linear model's weights [species][keys][props], the centre's
 // energy sum_P w P from the values on their way out (134 128 atoms: 0.72 ms;
-// 1.49 + 0.53 with a kernel that read them back).
+// 1.49 + 0.53 with a kernel that read them back): a lane's ten products of an l
+// and parity in T, their sums over l and lanes in FP64 (one sum of 140 terms in
+// FP32 was twice as far from the exact one as the 256-thread sums before it).
 template <typename T, bool ENERGY, int NT, bool N8>
 __global__ void __launch_bounds__(32 * DW_WARPS, 3)
 dense_contraction_tiles(DenseArgs<T> a, const T* __restrict__ weights, T* __restrict__ energy) {
@@ -164,10 +166,11 @@ dense_contraction_tiles(DenseArgs<T> a, const T* __restrict__ weights, T* __rest
     const T* X = a.coef + c * NT * (int64_t)K + N * t + (row ? g : 0);
     T* out = a.values + c * (NT * (NT + 1) / 2) * (int64_t)P + first;
     const T* w = ENERGY ? weights + (int64_t)a.atom_species[c] * (NT * (NT + 1) / 2) * P + first : nullptr;
-    T sum = T(0);
+    double sum = 0.0;
 #pragma unroll 1
     for (int l = 0; l <= a.lmax; l++) {
         const int M = 2 * l + 1;
+        T part[2] = {T(0), T(0)};  // of the energy
         T acc[NT + 1][NT][2];
 #pragma unroll
         for (int i = 0; i <= NT; i++)
@@ -195,24 +198,30 @@ dense_contraction_tiles(DenseArgs<T> a, const T* __restrict__ weights, T* __rest
                 const T v0 = acc[i][j][0] * scale, v1 = acc[i][j][1] * scale;
                 if (two) {
                     store2(out + key * P, v0, v1);
-                    if (ENERGY) sum += v0 * w[key * P] + v1 * w[key * P + 1];
+                    if (ENERGY) {
+                        part[0] += v0 * w[key * P];
+                        part[1] += v1 * w[key * P + 1];
+                    }
                 } else if (one) {
                     if (2 * t < N) {
                         out[key * P] = v0;
-                        if (ENERGY) sum += v0 * w[key * P];
+                        if (ENERGY) part[0] += v0 * w[key * P];
                     }
                     if (2 * t + 1 < N) {
                         out[key * P + 1] = v1;
-                        if (ENERGY) sum += v1 * w[key * P + 1];
+                        if (ENERGY) part[1] += v1 * w[key * P + 1];
                     }
                 }
             }
         out += N * N;
-        if (ENERGY) w += N * N;
+        if (ENERGY) {
+            w += N * N;
+            sum += (double)part[0] + (double)part[1];
+        }
     }
     if (ENERGY) {
         for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
-        if (lane == 0) energy[c] = sum;
+        if (lane == 0) energy[c] = (T)sum;
     }
 }
 
@@ -299,7 +308,7 @@ dense_contraction_warp(DenseArgs<T> a, const T* __restrict__ weights, T* __restr
     T* out_c = a.values + c * KP;
     const T* w_c = ENERGY ? weights + (int64_t)a.atom_species[c] * KP : nullptr;
     const bool pairs = (N & 1) == 0;  // two neighbouring columns are of one species, and 2-element aligned
-    T sum = T(0);
+    double sum = 0.0;  // of the energy
     for (int r0 = 0; r0 < SN; r0 += 32) {
         // columns from the row block's first species on
         for (int q0 = r0 / N * N / 32 * 32; q0 < SN; q0 += 32) {
@@ -366,6 +375,7 @@ dense_contraction_warp(DenseArgs<T> a, const T* __restrict__ weights, T* __restr
                 const T same = scales[l], other = scales[32 + l];
                 T* out = out_c + l * NN;
                 const T* w = ENERGY ? w_c + l * NN : nullptr;
+                T part[2] = {T(0), T(0)};
 #pragma unroll
                 for (int i = 0; i < 4; i++)
 #pragma unroll
@@ -377,26 +387,30 @@ dense_contraction_warp(DenseArgs<T> a, const T* __restrict__ weights, T* __restr
                             if (!(write & (1u << (4 * i + j)))) continue;
                             const T v1 = acc[i][j][1] * scale0;
                             store2(out + at, v0, v1);
-                            if (ENERGY) sum += v0 * w[at] + v1 * w[at + 1];
+                            if (ENERGY) {
+                                part[0] += v0 * w[at];
+                                part[1] += v1 * w[at + 1];
+                            }
                         } else {
                             if (write & (1u << (4 * i + j))) {
                                 out[at] = v0;
-                                if (ENERGY) sum += v0 * w[at];
+                                if (ENERGY) part[0] += v0 * w[at];
                             }
                             if (write & (1u << (16 + 4 * i + j))) {
                                 const int next = at + (crosses & (1u << j) ? P - N + 1 : 1);
                                 const T v1 = acc[i][j][1] * (equal & (1u << (16 + 4 * i + j)) ? same : other);
                                 out[next] = v1;
-                                if (ENERGY) sum += v1 * w[next];
+                                if (ENERGY) part[1] += v1 * w[next];
                             }
                         }
                     }
+                if (ENERGY) sum += (double)part[0] + (double)part[1];
             }
         }
     }
     if (ENERGY) {
         for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
-        if (lane == 0) energy[c] = sum;
+        if (lane == 0) energy[c] = (T)sum;
     }
 }
 

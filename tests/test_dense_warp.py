@@ -138,3 +138,26 @@ def test_large_bases_keep_fp32_products(atoms, species, max_radial, max_angular)
                 found = results[0][:, key, l * N * N:(l + 1) * N * N].double()
                 assert bool(((found - reference).abs() <= (2 * l + 3) * 2.0 ** -24 * size + 1e-40).all())
             key += 1
+
+
+def test_batch_energies_keep_small_terms():
+    """An atom's energy of 64 terms 1 (l = 0) and 2304 of 0.9 x 2^-25 (l > 0),
+    which an FP32 sum that runs on over l drops one by one (16 units of 2^-24 of
+    the sum).  With the sums over l in FP64 a term 1 is rounded once, the small
+    ones lose 2^-24 of themselves, and the energy is rounded once: 3 units."""
+    types = np.array(TYPES[:4], dtype=np.int32)
+    positions = torch.tensor([[0.0, 0.0, 0.0], [1.1, 0.2, 0.1], [0.1, 1.3, 0.4], [0.3, 0.5, 1.2]], dtype=torch.float64,
+                             device="cuda")
+    batch = torch_api.Batch(rb.SoapPowerSpectrum(**workloads.hypers(4.5, 7, 6)), [4], types, TYPES[:4])
+    batch.config = dict(batch.config, pipeline=1)
+    weights = torch.zeros((4, batch.n_keys, batch.n_properties), device="cuda")
+    values = batch.run(positions, batch.outputs(), weights=weights)["values"].reshape(weights.shape)
+    terms = torch.zeros_like(weights)
+    terms[0, 0, :64] = 1.0
+    terms[0, :, 64:] = 0.9 * 2.0 ** -25
+    used = (terms != 0) & (values.abs() > 1e-20)
+    weights[used] = terms[used] / values[used]
+    assert int(used.sum()) > 2300
+    energy = batch.run(positions, batch.outputs(), weights=weights)["energies"].double().cpu()
+    terms = values.double() * weights.double()
+    assert float((energy - terms.sum().cpu()).abs().max()) <= 3 * 2.0 ** -24 * float(terms.abs().sum())
