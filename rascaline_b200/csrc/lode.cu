@@ -325,7 +325,6 @@ namespace fb200 {
 
 namespace {
 
-constexpr int LODE_LCAP = 16;
 constexpr int LODE_KB = 16;       // k-vectors per step of the product, and the padding of their number
 constexpr int LODE_ROWS = 64;     // rows of one tile of the product
 constexpr int LODE_THREADS = 128;
@@ -703,7 +702,22 @@ __global__ void __launch_bounds__(256) lode_splits_kernel(LodeArgs a, int n_type
 // least 128 to a split, so that the CTAs fill whole waves of the chip: 1000
 // atoms have 336 CTAs for 592 places, and three splits of them, which fill
 // two thirds of the third wave, took 0.56 ms where the rule's choice takes
-// 0.51.  A split costs two steps (its prologue and its share of the sums).
+// 0.51.  A split costs two steps (its prologue and its share of the sums) and
+// the memory of the whole product, 512 MB of which are the most: more splits
+// than that holds gain a few percent of many waves (by the rule's own time 2 %
+// for 4500 k-vectors, up to 8 % for 19 200), and would take ten times the
+// output for 160 000 k-vectors.
+constexpr int64_t LODE_PARTIAL_BYTES = (int64_t)512 << 20;
+
+template <int NB, bool GRAD>
+int lode_resident() {
+    int device = 0, sms = 0, per_sm = 0;
+    CUDA_CHECK(cudaGetDevice(&device));
+    CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, lode_gemm_kernel<NB, GRAD>, LODE_THREADS, 0));
+    return sms * std::max(1, per_sm);
+}
+
 template <bool GRAD>
 void launch_lode_gemm(LodeArgs a, int64_t rows, int n_types, DeviceArena& arena, cudaStream_t stream) {
     if (rows == 0 || n_types == 0) return;
@@ -715,10 +729,12 @@ void launch_lode_gemm(LodeArgs a, int64_t rows, int n_types, DeviceArena& arena,
     a.tiles = a.tiles_even + tiles(8 * nb, a.cols.n_odd);
     const int64_t row_tiles = (rows + LODE_ROWS - 1) / LODE_ROWS;
     const int64_t ctas = row_tiles * a.tiles * n_types;
-    const int steps = a.Kp / LODE_KB, resident = 148 * (GRAD ? 3 : 4);
+    const int steps = a.Kp / LODE_KB, resident = nb == 7 ? lode_resident<7, GRAD>() : lode_resident<8, GRAD>();
+    const int64_t split_bytes = (int64_t)sizeof(double) * n_types * rows * a.cols.ld;
     int best = 1;
     double best_time = 1e300;
     for (int q = 1; q <= std::max(1, std::min(32, steps / 8)); q++) {
+        if (q > 1 && q * split_bytes > LODE_PARTIAL_BYTES) break;
         const int64_t waves = (ctas * q + resident - 1) / resident;
         const double time = (double)waves * ((steps + q - 1) / q + 2);
         if (time < 0.98 * best_time) {
@@ -729,7 +745,7 @@ void launch_lode_gemm(LodeArgs a, int64_t rows, int n_types, DeviceArena& arena,
     a.split_k = (steps + best - 1) / best * LODE_KB;
     a.splits = (a.Kp + a.split_k - 1) / a.split_k;
     if (row_tiles * a.tiles > 0x7fffffffLL) throw invalid_parameter("the LODE product is too large for one launch");
-    if (a.splits > 1) a.partial = arena.alloc<double>("lode.partial", (int64_t)a.splits * n_types * rows * a.cols.ld);
+    if (a.splits > 1) a.partial = (double*)arena.alloc_bytes("lode.partial", a.splits * split_bytes);
     const dim3 grid((unsigned)(row_tiles * a.tiles), (unsigned)n_types, (unsigned)a.splits);
     if (nb == 7) lode_gemm_kernel<7, GRAD><<<grid, LODE_THREADS, 0, stream>>>(a);
     else lode_gemm_kernel<8, GRAD><<<grid, LODE_THREADS, 0, stream>>>(a);

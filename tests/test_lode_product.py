@@ -44,3 +44,30 @@ def test_tile_edges(atoms, max_radial, max_angular, smearing, gradients):
         x = np.concatenate([pick(b).reshape(-1) for b in ours["blocks"]])
         y = np.concatenate([pick(b).reshape(-1) for b in reference["blocks"]])
         assert np.all(np.abs(x - y) <= 1e-10 * np.abs(y) + 1e-12 * np.max(np.abs(y)))
+
+
+def test_splits_memory():
+    """Splits of the k-vectors keep a partial sum each, 512 MB together at most:
+    49 344 atoms and 9605 k-vectors, whose waves seven splits of 155 MB would
+    fill best.  Beside them a call keeps its phases, table and output, and the
+    small arrays and the pool's granularity below 200 MB."""
+    torch = pytest.importorskip("torch")
+    hypers = {"density": {"type": "SmearedPowerLaw", "smearing": 1.0, "exponent": 1},
+              "basis": {"type": "TensorProduct", "max_angular": 6, "radial": {"type": "Gto", "max_radial": 7, "radius": 3.0}}}
+    cell = 27.7 * np.eye(3)
+    atoms, k, columns = 49344, 9616, 392
+
+    def run(n):
+        positions = np.random.default_rng(n).uniform(0.0, 27.7, (n, 3))
+        calculator = rb.LodeSphericalExpansion(**hypers)
+        system = rb.System.from_dict({"types": np.ones(n, dtype=np.int32), "positions": positions, "cell": cell})
+        return calculator, calculator.compute(system)
+
+    run(100)
+    before = torch.cuda.mem_get_info()[0]
+    calculator, result = run(atoms)
+    used = before - torch.cuda.mem_get_info()[0]
+    del result
+    assert calculator is not None
+    expected = 8 * (2 * atoms * k + k * columns + atoms * columns)
+    assert expected - (64 << 20) <= used <= expected + (512 << 20) + (200 << 20)
