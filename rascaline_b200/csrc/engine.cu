@@ -341,11 +341,15 @@ Engine::~Engine() {
 
 void* Engine::staging(size_t bytes) {
     if (bytes > staging_bytes_) {
+        // by a quarter at least, as the device's buffers grow: with positions
+        // gradients the size follows the pairs, which a trajectory has more of
+        // again and again
+        const size_t grow = std::max(bytes, staging_bytes_ + staging_bytes_ / 4);
         if (staging_) CUDA_CHECK(cudaFreeHost(staging_));
         staging_ = nullptr;
         staging_bytes_ = 0;
-        CUDA_CHECK(cudaHostAlloc(&staging_, bytes, cudaHostAllocDefault));
-        staging_bytes_ = bytes;
+        CUDA_CHECK(cudaHostAlloc(&staging_, grow, cudaHostAllocDefault));
+        staging_bytes_ = grow;
     }
     return staging_;
 }

@@ -45,3 +45,28 @@ def test_device_tables_give_the_rows_of_the_host_tables(system, cutoff, max_radi
         for g in gradients:
             np.testing.assert_array_equal(a["gradients"][g]["samples"], b["gradients"][g]["samples"])
             np.testing.assert_array_equal(a["gradients"][g]["values"], b["gradients"][g]["values"])
+
+
+def test_growing_neighbourhoods_keep_their_staging():
+    """Twenty steps of a box that shrinks, each with more pairs than the last:
+    the pinned buffer of the neighbourhood tables grows by a quarter at a time,
+    here once at most, where an exact size would be freed at every step."""
+    torch = pytest.importorskip("torch")
+    from torch.profiler import ProfilerActivity, profile
+
+    box = workloads.random_box(200, seed=1, species=(1, 8))
+    calculator = rb.SphericalExpansion(**workloads.hypers(4.0, 2, 1))
+
+    def step(k):
+        f = 1.0 - 0.002 * k
+        calculator.compute([workloads.system_dict(box["types"], np.asarray(box["positions"]) * f, np.asarray(box["cell"]) * f)],
+                           gradients=["positions"])
+
+    step(0)
+    torch.zeros(1, device="cuda")
+    with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as profiler:
+        for k in range(1, 21):
+            step(k)
+    calls = [e.name for e in profiler.events()]
+    assert any("LaunchKernel" in name for name in calls)
+    assert sum("FreeHost" in name for name in calls) <= 1
