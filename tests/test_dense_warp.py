@@ -161,3 +161,33 @@ def test_batch_energies_keep_small_terms():
     energy = batch.run(positions, batch.outputs(), weights=weights)["energies"].double().cpu()
     terms = values.double() * weights.double()
     assert float((energy - terms.sum().cpu()).abs().max()) <= 3 * 2.0 ** -24 * float(terms.abs().sum())
+
+
+@pytest.mark.parametrize("atoms,species,max_radial,max_angular", [
+    (30, 9, 7, 3), (20, 16, 7, 2), (17, 5, 12, 2), (12, 6, 15, 2), (25, 20, 7, 1),
+])
+def test_blocks_of_many_functions(atoms, species, max_radial, max_angular):
+    """65 to 160 (s, n): three to five blocks of 32, species that begin in one and
+    end in the next.  FP64 within 1e-12 of the sum of sizes, FP32
+    within 2e-6 of the largest value (as above), from the coefficients."""
+    types = np.random.default_rng(atoms).permutation([1 + k % species for k in range(atoms)])
+    system = workloads.random_box(atoms, seed=atoms, species=(1,))
+    positions, cell = torch.tensor(system["positions"], device="cuda"), np.asarray(system["cell"]).reshape(1, 9)
+    hypers = workloads.hypers(4.0, max_radial, max_angular)
+    N = max_radial + 1
+    for precision in (64, 32):
+        values, _ = torch_api.dense_power_spectrum(rb.SoapPowerSpectrum(**hypers), positions, types, cell, [atoms], precision)
+        c, _ = torch_api.dense_spherical_expansion(rb.SphericalExpansion(**hypers), positions, types, cell, [atoms], precision)
+        c = c.double().reshape(atoms, species, (max_angular + 1) ** 2, N)
+        largest = float(values.abs().max())
+        key = 0
+        for a in range(species):
+            for b in range(a, species):
+                for l in range(max_angular + 1):
+                    x, y = (c[:, s, l * l:(l + 1) ** 2] for s in (a, b))
+                    scale = (-1) ** l / np.sqrt(2 * l + 1) * (np.sqrt(2) if a != b else 1)
+                    reference = torch.einsum("cmp,cmq->cpq", x, y).reshape(atoms, -1) * scale
+                    size = torch.einsum("cmp,cmq->cpq", x.abs(), y.abs()).reshape(atoms, -1) * abs(scale)
+                    error = (values[:, key, l * N * N:(l + 1) * N * N].double() - reference).abs()
+                    assert bool((error <= (1e-12 * size + 1e-300 if precision == 64 else 2e-6 * largest)).all())
+                key += 1
