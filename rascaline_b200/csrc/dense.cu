@@ -901,6 +901,13 @@ void launch_dense_forward(const DenseArgs<T>& a, int64_t n_pairs, cudaStream_t s
         mark(3);
         return;
     }
+    if constexpr (sizeof(T) == 4) {
+        if (dense_mma_enabled() && dense_mma_supported(a) && (uintptr_t)a.values % 16 == 0) {
+            launch_dense_contraction_mma(a, stream);
+            mark(3);
+            return;
+        }
+    }
     const size_t smem = sizeof(T) * (size_t)a.n_species * a.K;
     if (a.nmax <= 16 && smem <= 48 * 1024) {
         if (a.nmax <= 8) dense_contraction_tiled<T, 8><<<(unsigned)a.n_atoms, 128, smem, stream>>>(a);

@@ -106,9 +106,11 @@ struct DenseState {
     std::vector<void*> allocations_;
 };
 
-// FP32 dL/dc on the tcgen05 tensor cores (dense_mma.cu), supported when
-// S nmax <= 128 and 2 lmax + 1 <= 32
+// FP32 contractions on the tcgen05 tensor cores (dense_mma.cu), supported when
+// S nmax <= 128 and 2 lmax + 1 <= 32 (the power spectrum: with 16-byte aligned
+// values)
 bool dense_mma_supported(const DenseArgs<float>& a);
+void launch_dense_contraction_mma(const DenseArgs<float>& a, cudaStream_t stream);
 void launch_dense_grad_coef_mma(const DenseArgs<float>& a, cudaStream_t stream);
 // angular channels per round of the tensor-core kernels (1 to 4)
 extern int dense_mma_channels_per_round;

@@ -1,18 +1,24 @@
-// dL/dc of the FP32 dense power spectrum on the sm_100a tensor cores
-// (tcgen05, TF32 operands split into hi + lo, FP32 accumulation in tensor
-// memory); the power spectrum itself and dL/dc of a linear model's batch are
-// in dense_warp.cu:
+// The two per-centre contractions of the FP32 dense power spectrum on the
+// sm_100a tensor cores (tcgen05, TF32 operands split into hi + lo, FP32
+// accumulation in tensor memory):
 //
-//   dL/dc_l[(a, n)][m] = sum_(b, q) G'_l[(a, n), (b, q)] X_l[m][(b, q)]
-//   with X_l[m][(s, n)] = c[s][l m][n] and G'_l the dL/dP block of the species
-//   pair (min, max) read as is (a < b), transposed (a > b) or symmetrised
-//   (a == b), times scale(l, a != b)
-//   (the adjoint of featomic's power_spectrum.rs:529-780)
+//   forward   P_l = X_l^T X_l,  X_l[m][(s, n)] = c[s][l m][n]
+//             P_ab[l][n1][n2] = scale(l, a != b) P_l[(a, n1), (b, n2)]
+//             (featomic's power_spectrum.rs:529-780); nmax <= 8 with at most
+//             four species has a kernel of its own (dense_warp.cu)
+//   adjoint   dL/dc_l[(a, n)][m] = sum_(b, q) G'_l[(a, n), (b, q)] X_l[m][(b, q)]
+//             with G'_l the dL/dP block of the species pair (min, max) read
+//             as is (a < b), transposed (a > b) or symmetrised (a == b),
+//             times scale(l, a != b)
 //
 // A tile is G = 128 / SNP centres, SNP = S nmax rounded up to 32, 64 or 128:
-// MMA row r = g SNP + s nmax + n; A = [G'_l of each centre] (rows r, K = (b, q)
-// rounded up to 8), B = [X_l of each centre, m padded to MP] (N = G MP rows):
-// D[(g, a, n), (g', m)] is dL/dc when g' = g.
+// MMA row r = g SNP + s nmax + n.
+//   forward  A = B = [X_l of the tile's centres]^T (rows r, K = m rounded up
+//            to 8): D = A B^T is 128 x 128 and the diagonal SNP x SNP blocks
+//            are the centres' P_l (the other blocks are not read).
+//   adjoint  A = [G'_l of each centre] (rows r, K = (b, q) rounded up to 8),
+//            B = [X_l of each centre, m padded to MP] (N = G MP rows):
+//            D[(g, a, n), (g', m)] is dL/dc when g' = g.
 // Every product is hi_a hi_b + hi_a lo_b + lo_a hi_b (three MMAs): the
 // dropped lo lo term is below 2^-22 of the product, so the results are
 // within a few FP32 ulps of the CUDA-core contractions.
@@ -32,6 +38,8 @@ namespace {
 
 constexpr int ROWS = 128;
 constexpr int THREADS = 256;
+
+__device__ __forceinline__ int kpad_l(int l) { return (2 * l + 1 + 7) & ~7; }
 
 // power spectrum normalisation 1 / ((-1)^l sqrt(2l + 1)), times sqrt(2) for
 // two different neighbour species, evaluated in FP64 and rounded like the
@@ -111,6 +119,122 @@ __device__ __forceinline__ bool round_wait(const Ctx& c, uint32_t& phase, int32_
     if (*abort_flag) return false;
     tc::fence_after();
     return true;
+}
+
+__global__ void __launch_bounds__(THREADS) dense_contraction_mma(DenseArgs<float> a, MmaShape sh) {
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    __shared__ uint64_t bar;
+    __shared__ uint32_t tmem_slot;
+    __shared__ int abort_flag;
+    __shared__ float scales[32];
+    if (threadIdx.x == 0) abort_flag = 0;
+    fill_scales(scales);
+    const Ctx ctx = setup(smem_raw, sh, &bar, &tmem_slot);
+    const int S = a.n_species, N = a.nmax, K = a.K, NN = N * N, lmax = a.lmax;
+    const int SN = sh.SN, SNP = sh.SNP, G = sh.G;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = warp & 3, half = warp >> 2;
+    const int64_t tiles = (a.n_atoms + G - 1) / G;
+    uint32_t phase = 0;
+    bool aborted = false;
+    // the operand row this thread builds: r = g SNP + s nmax + n
+    const int row = threadIdx.x & (ROWS - 1), kh = threadIdx.x >> 7;
+    const int row_g = row / SNP, row_rr = row - row_g * SNP;
+    const int row_s = row_rr / N, row_n = row_rr - row_s * N;
+    for (int64_t tile = blockIdx.x; tile < tiles && !aborted; tile += gridDim.x) {
+        const int64_t c0 = tile * G;
+        const int ng = (int)min((int64_t)G, a.n_atoms - c0);
+        const bool row_ok = row_g < ng && row_rr < SN;
+        const float* row_src = a.coef + ((c0 + (row_ok ? row_g : 0)) * S + row_s) * (int64_t)K + row_n;
+        for (int l0 = 0; l0 <= lmax; l0 += sh.lpr) {
+            const int l1 = min(lmax, l0 + sh.lpr - 1);
+            // operands: for each channel of the round, rows r, K = m padded
+            // to 8; thread = (row, half of the K quads)
+            int off = 0;
+            for (int l = l0; l <= l1; l++) {
+                const int kp = kpad_l(l), M = 2 * l + 1;
+                const float* src = row_src + (int64_t)l * l * N;
+                for (int k4 = kh; k4 < kp / 4; k4 += 2) {
+                    float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                    if (row_ok) {
+#pragma unroll
+                        for (int e = 0; e < 4; e++) {
+                            const int m = 4 * k4 + e;
+                            if (m < M) v[e] = __ldg(src + m * N);
+                        }
+                    }
+                    store_quad(ctx.hi, ctx.lo, off + tc::core_offset(row, 4 * k4, kp * 4, 4), v);
+                }
+                off += ROWS * kp * 4;
+            }
+            tc::fence_async_smem();
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                tc::fence_after();
+                const uint32_t idesc = tc::instr_desc(tc::FORMAT_TF32, ROWS, ROWS);
+                const uint32_t hi = tc::smem_addr(ctx.hi), lo = tc::smem_addr(ctx.lo);
+                int o = 0;
+                for (int l = l0; l <= l1; l++) {
+                    const int kp = kpad_l(l);
+                    const uint32_t sbo = (uint32_t)(kp / 4) * 128;
+                    const uint32_t d = ctx.tmem + (uint32_t)((l - l0) * ROWS);
+                    for (int ks = 0; ks < kp / 8; ks++) {
+                        const uint64_t ah = tc::operand_desc(hi + o + 256 * ks, 128, sbo);
+                        const uint64_t al = tc::operand_desc(lo + o + 256 * ks, 128, sbo);
+                        tc::mma_tf32(d, ah, ah, idesc, ks > 0);
+                        tc::mma_tf32(d, ah, al, idesc, 1);
+                        tc::mma_tf32(d, al, ah, idesc, 1);
+                    }
+                    o += ROWS * kp * 4;
+                }
+                tc::mma_commit(ctx.bar);
+            }
+            if (!round_wait(ctx, phase, a.status, &abort_flag)) {
+                aborted = true;
+                break;
+            }
+            // epilogue: warp (q, half) reads rows 32 q .. 32 q + 31 of its
+            // centre's diagonal block, 16 columns at a time
+            const int r = 32 * q + lane;
+            const int g = (32 * q) / SNP;
+            const int rr = r - g * SNP;
+            const int s = rr / N, n1 = rr - s * N;
+            const bool out_ok = g < ng && rr < SN;
+            const int chunks = (SN + 15) / 16;
+            const int items = (l1 - l0 + 1) * chunks;
+            for (int item = half; item < items; item += 2) {
+                const int j = item / chunks, ch = item - j * chunks;
+                const int l = l0 + j;
+                float v[16];
+                tc::tmem_load16(ctx.tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(j * ROWS + g * SNP + 16 * ch), v);
+                if (!out_ok) continue;
+                float* out = a.values + (c0 + g) * (int64_t)a.n_keys * a.n_props + (int64_t)l * NN + n1 * N;
+                if ((N & 3) == 0) {
+#pragma unroll
+                    for (int t = 0; t < 16; t += 4) {
+                        const int col = 16 * ch + t;
+                        const int sb = col / N, n2 = col - sb * N;
+                        if (col < SN && sb >= s) {
+                            const float sc = scales[(sb != s ? 16 : 0) + l];
+                            float* dst = out + (int64_t)key_of(s, sb, S) * a.n_props + n2;
+                            *reinterpret_cast<float4*>(dst) =
+                                make_float4(v[t] * sc, v[t + 1] * sc, v[t + 2] * sc, v[t + 3] * sc);
+                        }
+                    }
+                } else {
+#pragma unroll
+                    for (int t = 0; t < 16; t++) {
+                        const int col = 16 * ch + t;
+                        const int sb = col / N, n2 = col - sb * N;
+                        if (col < SN && sb >= s)
+                            out[(int64_t)key_of(s, sb, S) * a.n_props + n2] = v[t] * scales[(sb != s ? 16 : 0) + l];
+                    }
+                }
+            }
+            tc::fence_before();
+            __syncthreads();
+        }
+    }
+    teardown(ctx, sh, aborted, phase);
 }
 
 __global__ void __launch_bounds__(THREADS) dense_grad_coef_mma(DenseArgs<float> a, MmaShape sh) {
@@ -341,6 +465,28 @@ int dense_mma_channels_per_round = 1;
 
 bool dense_mma_supported(const DenseArgs<float>& a) {
     return a.n_atoms > 0 && a.n_species * a.nmax <= ROWS && 2 * a.lmax + 1 <= 32 && a.lmax < 16;
+}
+
+void launch_dense_contraction_mma(const DenseArgs<float>& a, cudaStream_t stream) {
+    MmaShape sh = base_shape(a);
+    sh.lpr = std::max(1, std::min(dense_mma_channels_per_round, 4));
+    // the largest round: sum of K paddings of lpr consecutive channels
+    auto round_k = [&](int lpr) {
+        int kmax = 0;
+        for (int l0 = 0; l0 <= a.lmax; l0 += lpr) {
+            int k = 0;
+            for (int l = l0; l <= std::min(a.lmax, l0 + lpr - 1); l++) k += (2 * l + 1 + 7) & ~7;
+            kmax = std::max(kmax, k);
+        }
+        return kmax;
+    };
+    // at most 200 KB of operands per round
+    while (sh.lpr > 1 && 2 * ROWS * round_k(sh.lpr) * 4 > 200 * 1024) sh.lpr--;
+    sh.tmem_cols = tmem_columns(sh.lpr * ROWS);
+    const int kmax = round_k(sh.lpr);
+    sh.region = ROWS * kmax * 4;
+    const int64_t tiles = (a.n_atoms + sh.G - 1) / sh.G;
+    launch_persistent(dense_contraction_mma, a, sh, 2 * (size_t)sh.region, tiles, stream);
 }
 
 void launch_dense_grad_coef_mma(const DenseArgs<float>& a, cudaStream_t stream) {

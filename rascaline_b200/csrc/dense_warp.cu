@@ -65,39 +65,14 @@ __device__ __forceinline__ void store2(float* p, float x, float y) { __stcs(rein
 __device__ __forceinline__ void store2(double* p, double x, double y) { __stcs(reinterpret_cast<double2*>(p), make_double2(x, y)); }
 
 // acc (4 x 4 tiles of 8 x 8, lane: row lane / 4, columns 2 (lane % 4) + {0, 1})
-// += the products of one step of m (8 in FP32, 4 in FP64): x, y [column tile]
-// hold rows m = lane % 4 (and + 4) at column lane / 4.  Tile (i, j) is
-// computed when bit 4 i + j of `need` is set.
-__device__ __forceinline__ void step(float (&acc)[4][4][2], const float (&x)[4][2], const float (&y)[4][2], unsigned need) {
-    uint32_t yh[4][2], yl[4][2];
-#pragma unroll
-    for (int j = 0; j < 4; j++)
-#pragma unroll
-        for (int e = 0; e < 2; e++) split(y[j][e], yh[j][e], yl[j][e]);
-#pragma unroll
-    for (int i = 0; i < 2; i++) {
-        uint32_t h[2][2], l[2][2];
-#pragma unroll
-        for (int q = 0; q < 2; q++)
-#pragma unroll
-            for (int e = 0; e < 2; e++) split(x[2 * i + q][e], h[q][e], l[q][e]);
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            if (!(need & (0x11u << (8 * i + j)))) continue;
-            float(&top)[2] = acc[2 * i][j];
-            float(&bottom)[2] = acc[2 * i + 1][j];
-            mma_tf32(top, bottom, h[0][0], h[1][0], h[0][1], h[1][1], yh[j][0], yh[j][1]);
-            mma_tf32(top, bottom, h[0][0], h[1][0], h[0][1], h[1][1], yl[j][0], yl[j][1]);
-            mma_tf32(top, bottom, l[0][0], l[1][0], l[0][1], l[1][1], yh[j][0], yh[j][1]);
-        }
-    }
-}
-__device__ __forceinline__ void step(double (&acc)[4][4][2], const double (&x)[4][1], const double (&y)[4][1], unsigned need) {
+// += the products of four m: x, y [column tile] hold rows m = lane % 4 at column
+// lane / 4.  Tile (i, j) is computed when bit 4 i + j of `need` is set.
+__device__ __forceinline__ void step(double (&acc)[4][4][2], const double (&x)[4], const double (&y)[4], unsigned need) {
 #pragma unroll
     for (int i = 0; i < 4; i++)
 #pragma unroll
         for (int j = 0; j < 4; j++)
-            if (need & (1u << (4 * i + j))) mma_f64(acc[i][j], x[i][0], y[j][0]);
+            if (need & (1u << (4 * i + j))) mma_f64(acc[i][j], x[i], y[j]);
 }
 
 // One step of m (8 in FP32, 4 in FP64) of the upper tiles (i <= j < NT) of
@@ -285,18 +260,12 @@ dense_tangent_tiles(DenseArgs<T> a, const T* __restrict__ tcoef, T* __restrict__
     }
 }
 
-// The same for any nmax and number of species, by blocks of 32 x 32 (s, n).
-// What depends on a row or column alone is found once per block: an offset
-// among the values is a row's term plus a column's.  (With the divisions by
-// nmax in the loop over m it lost to the tcgen05 tiles for 33 to 64 (s, n).)
-// FP32 forward pass of 20 000 atoms, 4 species, nmax 12, lmax 8: 3.10 ms, 4.55
-// with the divisions, 4.16 on tcgen05; 4000 atoms, nmax 16, lmax 6: 0.58 ms,
-// 0.87 and 0.80.
-template <typename T, bool ENERGY>
-__global__ void __launch_bounds__(32 * DW_WARPS, 2)
-dense_contraction_warp(DenseArgs<T> a, const T* __restrict__ weights, T* __restrict__ energy) {
-    constexpr int E = sizeof(T) == 4 ? 2 : 1, STEP = 4 * E;
-    __shared__ T scales[64];
+// The values in FP64 for any nmax and number of species, by blocks of 32 x 32
+// (s, n); dense_contraction_by_warp says where.  What depends on a row or column
+// alone is found once per block: an offset among the values is a row's term plus
+// a column's.
+__global__ void __launch_bounds__(32 * DW_WARPS, 2) dense_contraction_warp(DenseArgs<double> a) {
+    __shared__ double scales[64];
     fill_scales(scales);
     __syncthreads();
     const int lane = threadIdx.x & 31, t = lane & 3, g = lane >> 2;
@@ -304,11 +273,9 @@ dense_contraction_warp(DenseArgs<T> a, const T* __restrict__ weights, T* __restr
     if (c >= a.n_atoms) return;
     const int S = a.n_species, N = a.nmax, K = a.K, SN = S * N, NN = N * N, P = (int)a.n_props;
     const int64_t KP = (int64_t)a.n_keys * P;
-    const T* X = a.coef + c * S * (int64_t)K;
-    T* out_c = a.values + c * KP;
-    const T* w_c = ENERGY ? weights + (int64_t)a.atom_species[c] * KP : nullptr;
+    const double* X = a.coef + c * S * (int64_t)K;
+    double* out_c = a.values + c * KP;
     const bool pairs = (N & 1) == 0;  // two neighbouring columns are of one species, and 2-element aligned
-    double sum = 0.0;  // of the energy
     for (int r0 = 0; r0 < SN; r0 += 32) {
         // columns from the row block's first species on
         for (int q0 = r0 / N * N / 32 * 32; q0 < SN; q0 += 32) {
@@ -350,67 +317,46 @@ dense_contraction_warp(DenseArgs<T> a, const T* __restrict__ weights, T* __restr
 #pragma unroll 1
             for (int l = 0; l <= a.lmax; l++) {
                 const int M = 2 * l + 1;
-                T acc[4][4][2];
+                double acc[4][4][2];
 #pragma unroll
                 for (int i = 0; i < 4; i++)
 #pragma unroll
-                    for (int j = 0; j < 4; j++) acc[i][j][0] = acc[i][j][1] = T(0);
+                    for (int j = 0; j < 4; j++) acc[i][j][0] = acc[i][j][1] = 0.0;
 #pragma unroll 1
-                for (int m0 = 0; m0 < M; m0 += STEP) {
-                    T x[4][E], y[4][E];
+                for (int m0 = 0; m0 < M; m0 += 4) {
+                    double x[4], y[4];
+                    const int m = m0 + t;
+                    const double* row = X + (l * l + m) * N;
+                    const bool ok = m < M;
 #pragma unroll
-                    for (int e = 0; e < E; e++) {
-                        const int m = m0 + t + 4 * e;
-                        const T* row = X + (l * l + m) * N;
-                        const bool ok = m < M;
-#pragma unroll
-                        for (int i = 0; i < 4; i++) {
-                            x[i][e] = ok && x_at[i] >= 0 ? __ldg(row + x_at[i]) : T(0);
-                            if (!diagonal) y[i][e] = ok && y_at[i] >= 0 ? __ldg(row + y_at[i]) : T(0);
-                        }
+                    for (int i = 0; i < 4; i++) {
+                        x[i] = ok && x_at[i] >= 0 ? __ldg(row + x_at[i]) : 0.0;
+                        if (!diagonal) y[i] = ok && y_at[i] >= 0 ? __ldg(row + y_at[i]) : 0.0;
                     }
                     if (diagonal) step(acc, x, x, need);
                     else step(acc, x, y, need);
                 }
-                const T same = scales[l], other = scales[32 + l];
-                T* out = out_c + l * NN;
-                const T* w = ENERGY ? w_c + l * NN : nullptr;
-                T part[2] = {T(0), T(0)};
+                const double same = scales[l], other = scales[32 + l];
+                double* out = out_c + l * NN;
 #pragma unroll
                 for (int i = 0; i < 4; i++)
 #pragma unroll
                     for (int j = 0; j < 4; j++) {
                         const int at = row_at[i] + column_at[j];
-                        const T scale0 = equal & (1u << (4 * i + j)) ? same : other;
-                        const T v0 = acc[i][j][0] * scale0;
+                        const double scale0 = equal & (1u << (4 * i + j)) ? same : other;
+                        const double v0 = acc[i][j][0] * scale0;
                         if (pairs) {
                             if (!(write & (1u << (4 * i + j)))) continue;
-                            const T v1 = acc[i][j][1] * scale0;
-                            store2(out + at, v0, v1);
-                            if (ENERGY) {
-                                part[0] += v0 * w[at];
-                                part[1] += v1 * w[at + 1];
-                            }
+                            store2(out + at, v0, acc[i][j][1] * scale0);
                         } else {
-                            if (write & (1u << (4 * i + j))) {
-                                out[at] = v0;
-                                if (ENERGY) part[0] += v0 * w[at];
-                            }
-                            if (write & (1u << (16 + 4 * i + j))) {
-                                const int next = at + (crosses & (1u << j) ? P - N + 1 : 1);
-                                const T v1 = acc[i][j][1] * (equal & (1u << (16 + 4 * i + j)) ? same : other);
-                                out[next] = v1;
-                                if (ENERGY) part[1] += v1 * w[next];
-                            }
+                            if (write & (1u << (4 * i + j))) out[at] = v0;
+                            if (write & (1u << (16 + 4 * i + j)))
+                                out[at + (crosses & (1u << j) ? P - N + 1 : 1)] =
+                                    acc[i][j][1] * (equal & (1u << (16 + 4 * i + j)) ? same : other);
                         }
                     }
-                if (ENERGY) sum += (double)part[0] + (double)part[1];
             }
         }
-    }
-    if (ENERGY) {
-        for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
-        if (lane == 0) energy[c] = (T)sum;
     }
 }
 
@@ -583,18 +529,27 @@ __global__ void __launch_bounds__(32 * DW_WARPS) dense_grad_coef_species(DenseAr
     }
 }
 
+// a tile per species pair
+template <typename T>
+bool dense_tiles(const DenseArgs<T>& a) {
+    return a.nmax <= 8 && a.n_species <= 4;
+}
+
 }  // namespace
 
 template <typename T>
 bool dense_contraction_by_warp(const DenseArgs<T>& a) {
-    // two values are stored at a time
-    if (sizeof(T) == 8) return a.lmax < 32 && (uintptr_t)a.values % 16 == 0;
-    // FP32 as the CUDA cores' contraction where that is asked for, and where the
-    // tensor cores' dL/dc does not follow: FP32 multiply-adds are four times as
-    // close to the exact products as TF32 operands split into hi + lo (3.7e-8
-    // against 1.3e-7 of the norm)
-    if constexpr (sizeof(T) == 4) return dense_mma_enabled() && dense_mma_supported(a) && (uintptr_t)a.values % 16 == 0;
-    return false;
+    // two values are stored at a time, and the FP32 forms have one rule
+    if ((uintptr_t)a.values % 16 != 0 || a.lmax >= 32) return false;
+    if constexpr (sizeof(T) == 4) {
+        // FP32 as the CUDA cores' contraction where that is asked for, and from
+        // l = 16 on; larger bases keep the tcgen05 tiles, or the CUDA cores
+        // (a warp per centre lost to tcgen05 with more than 32 (s, n): 8000
+        // atoms, 6 species, nmax 8 271 against 224 us, 16 species 441 against
+        // 308, 300 atoms 99 against 26)
+        return dense_mma_enabled() && a.lmax < 16 && dense_tiles(a);
+    }
+    return true;
 }
 template bool dense_contraction_by_warp<float>(const DenseArgs<float>&);
 template bool dense_contraction_by_warp<double>(const DenseArgs<double>&);
@@ -612,13 +567,11 @@ void launch_dense_contraction_warp(const DenseArgs<T>& a, cudaStream_t stream) {
             default: run(dense_contraction_tiles<T, EN, 4, N8>); break;
         }
     };
-    if (a.nmax <= 8 && a.n_species <= 4) {
+    if (dense_tiles(a)) {
         if (a.nmax == 8) a.energy ? tiles(std::true_type(), std::true_type()) : tiles(std::false_type(), std::true_type());
         else a.energy ? tiles(std::true_type(), std::false_type()) : tiles(std::false_type(), std::false_type());
-    } else if (a.energy) {
-        run(dense_contraction_warp<T, true>);
     } else {
-        run(dense_contraction_warp<T, false>);
+        if constexpr (sizeof(T) == 8) dense_contraction_warp<<<blocks, 32 * DW_WARPS, 0, stream>>>(a);
     }
     CUDA_CHECK(cudaGetLastError());
 }
