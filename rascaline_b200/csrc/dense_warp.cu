@@ -549,7 +549,21 @@ bool dense_contraction_by_warp(const DenseArgs<T>& a) {
         // 308, 300 atoms 99 against 26)
         return dense_mma_enabled() && a.lmax < 16 && dense_tiles(a);
     }
-    return true;
+    // FP64.  A warp walks over all of a centre's l one after the other, which
+    // takes enough centres to hide: the tiles lose to the four warps a centre of
+    // dense.cu with l > 8 and few centres (30 atoms, 4 species, lmax 12 34
+    // against 26 us, 3000 atoms 81 against 222), the blocks of 32 with fewer
+    // than some 1000 centres (300 atoms, 10 species, nmax 14 222 against 85 us).
+    // Blocks also lose to them with many idle rows or odd 8-byte accesses (8000
+    // atoms, 5 species, nmax 8 306 against 267; nmax 5 460 against 253), and win
+    // with full ones (8000 atoms, 4 species, nmax 16 218 against 464) and where a
+    // centre's coefficients do not fit dense.cu's 48 KB (1200 atoms, 12 species,
+    // lmax 9 319 against 622).
+    if (dense_tiles(a)) return a.lmax <= 8 || a.n_atoms >= 2000;
+    const int SN = a.n_species * a.nmax, blocks = (SN + 31) / 32;
+    const bool full = a.nmax % 8 == 0 && 5 * SN >= 4 * 32 * blocks;
+    const bool staged = a.nmax <= 16 && sizeof(T) * (size_t)a.n_species * a.K <= 48 * 1024;
+    return a.n_atoms >= 1200 && (full || !staged);
 }
 template bool dense_contraction_by_warp<float>(const DenseArgs<float>&);
 template bool dense_contraction_by_warp<double>(const DenseArgs<double>&);

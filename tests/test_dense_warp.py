@@ -191,3 +191,30 @@ def test_blocks_of_many_functions(atoms, species, max_radial, max_angular):
                     error = (values[:, key, l * N * N:(l + 1) * N * N].double() - reference).abs()
                     assert bool((error <= (1e-12 * size + 1e-300 if precision == 64 else 2e-6 * largest)).all())
                 key += 1
+
+
+@pytest.mark.parametrize("atoms,species,max_radial,max_angular", [
+    (1199, 4, 7, 1), (1200, 4, 15, 1), (1199, 4, 15, 1), (1200, 5, 7, 1), (2000, 1, 2, 9), (1999, 1, 2, 9),
+])
+def test_fp64_on_both_sides_of_its_rule(atoms, species, max_radial, max_angular):
+    """The number of atoms, the fill of the blocks of 32 and lmax decide which
+    kernel makes the FP64 values: within 1e-12 of the sum of sizes on both
+    sides, from the coefficients."""
+    system = workloads.random_box(atoms, seed=atoms, species=TYPES[:species])
+    positions, cell = torch.tensor(system["positions"], device="cuda"), np.asarray(system["cell"]).reshape(1, 9)
+    hypers = workloads.hypers(2.5, max_radial, max_angular)
+    values, _ = torch_api.dense_power_spectrum(rb.SoapPowerSpectrum(**hypers), positions, system["types"], cell, [atoms], 64)
+    c, _ = torch_api.dense_spherical_expansion(rb.SphericalExpansion(**hypers), positions, system["types"], cell, [atoms], 64)
+    N = max_radial + 1
+    c = c.reshape(atoms, species, (max_angular + 1) ** 2, N)
+    key = 0
+    for a in range(species):
+        for b in range(a, species):
+            for l in range(max_angular + 1):
+                x, y = (c[:, s, l * l:(l + 1) ** 2] for s in (a, b))
+                scale = (-1) ** l / np.sqrt(2 * l + 1) * (np.sqrt(2) if a != b else 1)
+                reference = torch.einsum("cmp,cmq->cpq", x, y).reshape(atoms, -1) * scale
+                size = torch.einsum("cmp,cmq->cpq", x.abs(), y.abs()).reshape(atoms, -1) * abs(scale)
+                found = values[:, key, l * N * N:(l + 1) * N * N]
+                assert bool(((found - reference).abs() <= 1e-12 * size + 1e-300).all())
+            key += 1
