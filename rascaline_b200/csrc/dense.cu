@@ -992,10 +992,7 @@ template <typename T>
 void launch_dense_jvp(const DenseArgs<T>& a, int64_t n_pairs, const T* tangent_positions, const T* tangent_cell,
                       T* pair_tangent, T* tangent_coef, T* tangent_values, cudaStream_t stream) {
     if (a.n_atoms == 0) return;
-    // Wherever the coefficients are made by centre, so is their tangent: 1.2 to
-    // 3 times as fast with the contraction for 60 to 6000 atoms, nmax 4 to 12,
-    // lmax 3 to 9, both precisions (46 us against 57 at the smallest).
-    const bool by_centre = a.surrogate == nullptr && centre_expansion_supported(a.tab);
+    const bool by_centre = a.surrogate == nullptr && dense_tangent_by_centre(a.tab, a.n_atoms, n_pairs);
     if (by_centre) {
         launch_dense_tangent_by_centre(a, tangent_positions, tangent_cell, tangent_coef, stream);
     } else if (n_pairs > 0) {

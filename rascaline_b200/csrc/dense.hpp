@@ -132,11 +132,14 @@ void launch_dense_grad_coef_species(const DenseArgs<float>& a, cudaStream_t stre
 // tiles (species, first, count) over `order`, the atoms sorted by species
 std::vector<int32_t> dense_species_tiles(const std::vector<int32_t>& species, int n_species, std::vector<int32_t>& order);
 
-// tangent of the coefficients with one CTA per centre (dense_tangent.cu)
+// tangent of the coefficients with one CTA per centre (dense_tangent.cu), and
+// where it takes the place of the pair records (without a surrogate)
+template <typename T>
+bool dense_tangent_by_centre(const DenseTables<T>& tables, int64_t n_atoms, int64_t n_pairs);
 template <typename T>
 void launch_dense_tangent_by_centre(const DenseArgs<T>& a, const T* tpos, const T* tcell, T* tcoef, cudaStream_t stream);
 // tangent of the power spectrum with a warp per centre (nmax <= 8, at most
-// four species, 2-value alignment of tvalues)
+// four species, 2-value alignment of tvalues; not for few centres with l > 8)
 template <typename T>
 bool dense_tangent_by_warp(const DenseArgs<T>& a, const T* tvalues);
 template <typename T>

@@ -223,6 +223,31 @@ __global__ void __launch_bounds__(CE_THREADS) centre_tangent_kernel(DenseArgs<T>
 
 }  // namespace
 
+// Few directions: one launch instead of three, whatever the basis (500 atoms with
+// 38 directions 1.0 to 2.4 times as fast).  Many: the pair records' kernels have
+// a thread for every (pair, l, m), and a row of few coefficients does not hide
+// this kernel's chain of recursions and barriers.  `work` grows with the sums of
+// a direction; 4000 to 8000 atoms with 38 directions, pair records / by centre:
+//   FP32  lmax 1, nmax 4 (work 32) 85 / 116 us; 2, 4 (72) 0.9 times as fast;
+//         1, 16 (80) 1.02 to 1.07 times; 3, 4 (128) 1.2 to 1.3
+//   FP64  lmax 1, nmax 4 (32) 119 / 233 us; 3, 4 (128) 232 / 278; 2, 12 (144) 0.92;
+//         2, 16 (180) 1.1 to 1.3; 3, 8 (192) 1.1; 4, 4 (200) 1.2
+// With 11 directions a centre, a third of a chunk, FP64 turns at about 250 (lmax
+// 4, nmax 4 0.87 to 0.94, nmax 8 1.27).  Layouts of more than 112 KB (FP64, lmax 8,
+// nmax 15 and 16) leave one CTA of two warps per SM (0.9 to 0.97).
+template <typename T>
+bool dense_tangent_by_centre(const DenseTables<T>& tables, int64_t n_atoms, int64_t n_pairs) {
+    if (!centre_expansion_supported(tables)) return false;
+    constexpr bool F32 = sizeof(T) == 4;
+    if (2 * n_pairs <= (F32 ? 40000 : 24000)) return true;
+    const int L = tables.ylm_const.lmax, N = tables.spline.nmax, work = (L + 1) * (L + 1) * (N + 4);
+    if (work < (F32 ? 76 : 2 * n_pairs < 16 * n_atoms ? 250 : 175)) return false;
+    return TangentLayout<T>(L, N, tables.spline.levels).bytes <= 112 * 1024;
+}
+
+template bool dense_tangent_by_centre<float>(const DenseTables<float>&, int64_t, int64_t);
+template bool dense_tangent_by_centre<double>(const DenseTables<double>&, int64_t, int64_t);
+
 template <typename T>
 void launch_dense_tangent_by_centre(const DenseArgs<T>& a, const T* tpos, const T* tcell, T* tcoef, cudaStream_t stream) {
     const TangentLayout<T> lay(a.lmax, a.nmax, a.tab.spline.levels);

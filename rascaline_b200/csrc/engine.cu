@@ -1231,8 +1231,8 @@ void Engine::jvp_dense(DenseState& st, const void* tangent_positions, const void
     const int64_t P = st.n_pairs;
     const FeatureLayout layout = FeatureLayout::make(h_.max_angular, h_.nmax(), true);
     // the tangent by centre needs no pair records
-    const bool records = st.precision == 32 ? active_surrogate_ != nullptr || !centre_expansion_supported(dense_f_)
-                                            : !centre_expansion_supported(dense_d_);
+    const bool records = st.precision == 32 ? active_surrogate_ != nullptr || !dense_tangent_by_centre(dense_f_, st.n_atoms, P)
+                                            : !dense_tangent_by_centre(dense_d_, st.n_atoms, P);
     void* features = nullptr;
     void* pair_tangent = nullptr;
     if (records) {

@@ -109,3 +109,26 @@ def test_contraction_in_64_bits(species, max_radial, max_angular):
                 found = tangent[:, key, l * N * N:(l + 1) * N * N].double()
                 assert bool(((found - reference).abs() <= 2.0 ** -24 * reference.abs() + 2.0 ** -48 * size).all())
             key += 1
+
+
+@pytest.mark.parametrize("atoms,max_radial,max_angular", [
+    (600, 1, 1), (700, 1, 1), (700, 7, 3), (700, 3, 3), (1000, 3, 1), (1100, 3, 1), (1100, 7, 2),
+])
+def test_both_sides_of_the_rule(atoms, max_radial, max_angular):
+    """Around 24 000 (FP64) and 40 000 (FP32) directions, bases below and above
+    the line: the same bounds as above, whichever way the tangent goes."""
+    box = workloads.random_box(atoms, seed=atoms, species=TYPES[:2])
+    calculator = rb.SoapPowerSpectrum(**workloads.hypers(4.5, max_radial, max_angular))
+    positions, cell = torch.tensor(box["positions"], device="cuda"), np.asarray(box["cell"]).reshape(1, 9)
+    generator = torch.Generator().manual_seed(4)
+    move = torch.randn((atoms, 3), dtype=torch.float64, generator=generator).cuda()
+    strain = torch.randn((1, 3, 3), dtype=torch.float64, generator=generator).cuda()
+    values, state = torch_api.dense_power_spectrum(calculator, positions, box["types"], cell, [atoms], 64)
+    exact, _ = torch_api.dense_jvp(state, move, strain)
+    gradient = torch.randn(values.shape, dtype=torch.float64, generator=generator).cuda()
+    at_positions, _, at_cell = torch_api.dense_backward(state, gradient, 1, strain=False, cell=True)
+    left, right = float((gradient * exact).sum()), float((at_positions * move).sum() + (at_cell * strain).sum())
+    assert abs(left - right) <= 1e-12 * float((gradient.abs() * exact.abs()).sum())
+    _, state = torch_api.dense_power_spectrum(calculator, positions, box["types"], cell, [atoms], 32)
+    fast, _ = torch_api.dense_jvp(state, move.float(), strain.float())
+    assert float((fast.double() - exact).abs().max()) <= 2e-5 * float(exact.abs().max())
