@@ -485,12 +485,14 @@ const SparseCg& sparse_cg(int l1, int l2, int lambda) {
     return cache.emplace(std::make_tuple(l1, l2, lambda), std::move(sp)).first->second;
 }
 
+int64_t cg_table_rows(int l1, int lambda) { return (int64_t)(2 * lambda + 1) * ((2 * l1 + 1 + 3) / 4 * 4); }
+
 // The table of one (l1, l2, lambda) for the tensor-core kernel: per mu and m1
 // (padded to a multiple of 4) its two terms; false when an m1 has more.
 bool cg_coef_rows(const SparseCg& sp, int l1, int lambda, std::vector<CgCoef>& table) {
     const int pad = (2 * l1 + 1 + 3) / 4 * 4;
     const size_t base = table.size();
-    table.resize(base + (size_t)(2 * lambda + 1) * pad, CgCoef{});
+    table.resize(base + (size_t)cg_table_rows(l1, lambda), CgCoef{});
     for (int mu = 0; mu <= 2 * lambda; mu++)
         for (int e = sp.mu_starts[mu]; e < sp.mu_starts[mu + 1]; e++) {
             const CgEntry& x = sp.entries[e];
@@ -508,11 +510,47 @@ bool cg_coef_rows(const SparseCg& sp, int l1, int lambda, std::vector<CgCoef>& t
     return true;
 }
 
+bool cg_vector_stores(const featomic_b200_cg_task_t& t) {
+    const int64_t stride = t.output_stride == 0 ? (int64_t)t.n_first * t.n_second : t.output_stride;
+    return t.n_second % 2 == 0 && stride % 2 == 0 && reinterpret_cast<uintptr_t>(t.output) % 16 == 0;
+}
+
+// Whether the tensor cores are worth it: all tasks of more than 16 properties on
+// a side (with two or fewer 8-wide tiles a side the row loop's own work is not
+// covered by the DMMAs; 2000 centres, l <= 4: 24 x 24 properties, l <= 3, 0.33
+// against 0.58 ms; 16 x 16 0.63 against 0.56 ms; 8 x 8 0.53 against 0.30 ms), and
+// enough output for their tables.  Those are larger than the thread kernel's
+// lists, are made and copied by the host (l <= 6: 456 KB, 107 us of a call of 350),
+// and pay when the device has work to cover it with: 2500 times their size in
+// outputs that take 16-byte stores (l <= 2, 32 x 32 properties, 30 samples 42.7
+// against 45.8 us with the tables, 300 samples 66.9 and 46.7; l <= 6, 30 samples
+// 350 and 457, 100 samples 541 and 456); the thread kernel is slower with others,
+// for which 1000 times are enough (17 x 17, l <= 6: 100 samples 400 and 458, 300
+// samples 882 and 595), and 60 times tables of up to 16 KB (20 x 33, l <= 2: 10
+// samples 54 and 46).
+bool cg_product_mma_pays(const featomic_b200_cg_task_t* tasks, size_t n_tasks) {
+    std::vector<uint64_t> orders;
+    int64_t out = 0;
+    bool vector = true;
+    for (size_t i = 0; i < n_tasks; i++) {
+        const auto& t = tasks[i];
+        const int64_t items = t.n_samples * (int64_t)t.n_first * t.n_second;
+        if (items == 0) continue;
+        if (t.n_first <= 16 || t.n_second <= 16) return false;
+        out += items * (2 * t.lambda + 1) * (int64_t)sizeof(double);
+        vector = vector && cg_vector_stores(t);
+        orders.push_back((uint64_t)t.l1 << 40 | (uint64_t)t.l2 << 20 | (uint64_t)t.lambda);
+    }
+    std::sort(orders.begin(), orders.end());
+    orders.erase(std::unique(orders.begin(), orders.end()), orders.end());
+    int64_t table = 0;
+    for (uint64_t o : orders) table += cg_table_rows((int)(o >> 40), (int)(o & 0xfffff)) * (int64_t)sizeof(CgCoef);
+    const int64_t times = vector ? 2500 : table > 16 * 1024 ? 1000 : 60;
+    return out >= times * (table + 6000);  // 6000: what the other host work of a call is worth
+}
+
 // FP64 products on the tensor cores; false (nothing launched) when one of the
-// tasks does not fit the kernel, or has fewer than 17 properties on a side:
-// with two or fewer 8-wide tiles a side the row loop's own work is not
-// covered by the DMMAs (2000 centres, l <= 4: 24 x 24 properties, l <= 3, 0.33
-// against 0.58 ms; 16 x 16 0.63 against 0.56 ms; 8 x 8 0.53 against 0.30 ms).
+// tasks does not fit the kernel.
 bool cg_product_mma(const featomic_b200_cg_task_t* tasks, size_t n_tasks, cudaStream_t stream) {
     std::vector<DeviceCgGroup> groups;
     std::vector<CgRow> rows;
@@ -524,7 +562,6 @@ bool cg_product_mma(const featomic_b200_cg_task_t* tasks, size_t n_tasks, cudaSt
         const auto& t = tasks[i];
         const int64_t pq = (int64_t)t.n_first * t.n_second;
         if (t.n_samples * pq == 0) continue;
-        if (t.n_first <= 16 || t.n_second <= 16) return false;
         const int64_t stride = t.output_stride == 0 ? pq : t.output_stride;
         auto at = known.find({t.l1, t.l2, t.lambda});
         if (at == known.end()) {
@@ -532,7 +569,7 @@ bool cg_product_mma(const featomic_b200_cg_task_t* tasks, size_t n_tasks, cudaSt
             if (!cg_coef_rows(sparse_cg(t.l1, t.l2, t.lambda), t.l1, t.lambda, table)) return false;
             at = known.emplace(std::make_tuple(t.l1, t.l2, t.lambda), start).first;
         }
-        const bool vector = t.n_second % 2 == 0 && stride % 2 == 0 && reinterpret_cast<uintptr_t>(t.output) % 16 == 0;
+        const bool vector = cg_vector_stores(t);
         const int pad = (2 * t.l1 + 1 + 3) / 4 * 4;
         bool joins = false;
         if (!groups.empty()) {
@@ -606,7 +643,7 @@ void cg_product(const featomic_b200_cg_task_t* tasks, size_t n_tasks, int precis
             throw invalid_parameter("output_stride of Clebsch-Gordan task " + std::to_string(i) +
                                     " is smaller than n_first * n_second");
     }
-    if (precision == 64 && cg_product_mma(tasks, n_tasks, stream)) return;
+    if (precision == 64 && cg_product_mma_pays(tasks, n_tasks) && cg_product_mma(tasks, n_tasks, stream)) return;
     std::vector<DeviceCgTask> dev;
     std::vector<CgEntry> entries;
     std::vector<int32_t> mu_starts;
