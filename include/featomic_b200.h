@@ -328,15 +328,23 @@ featomic_status_t featomic_b200_dense_jvp(featomic_b200_dense_t* state, const vo
                                           const void* tangent_cell, void* tangent_coefficients, void* tangent_values,
                                           void* stream);
 
-/* Engine of the FP32 per-centre contractions of the dense forms (the power
- * spectrum P_l = X_l^T X_l and the adjoint dL/dc): `tensor_cores` = 1 (the
- * default) runs them on the tcgen05 tensor cores with TF32 hi + lo operands
- * and FP32 accumulation, 0 on the CUDA cores; the value of the environment
- * variable FEATOMIC_B200_DENSE_MMA ("0" or "1") is the initial setting.
- * Process-wide; FP64 always uses the CUDA cores.  `channels_per_round`
- * (1 to 4, or 0 to keep the current value) is the number of angular channels
- * of one tensor-core round; FEATOMIC_B200_MMA_CHANNELS gives its initial
- * value.  No counterpart in featomic. */
+/* Engine of the FP32 per-centre contractions of the dense forms: the power
+ * spectrum P_l = X_l^T X_l, its tangent and the adjoint dL/dc.  `tensor_cores` =
+ * 1 (the default) runs them on the tensor cores, 0 on the CUDA cores with FP32
+ * multiply-adds; the value of the environment variable FEATOMIC_B200_DENSE_MMA
+ * ("0" or "1") is the initial setting.  On the tensor cores the power spectrum
+ * of up to 8 radial functions and 4 types is made by a warp per centre
+ * (mma.sync), that of more, up to 128 (types x radial functions) and
+ * max_angular < 16, on tcgen05 tiles, as is dL/dc with a row of dL/dP per atom;
+ * a batch's dL/dc with a row per type takes mma.sync.  Operands are TF32 split
+ * into hi + lo, sums FP32; the tangent (up to 8 radial functions and 4 types) is
+ * multiplied and summed in FP64.  Everything larger uses the CUDA cores.
+ * Process-wide.  The setting does not reach FP64, which takes the FP64 tensor
+ * cores or the CUDA cores by size (the same products, added in another order).
+ * `channels_per_round` (1 to 4, or 0 to keep the current value) is the number of
+ * angular channels of one round of the tcgen05 kernels;
+ * FEATOMIC_B200_MMA_CHANNELS gives its initial value.  No counterpart in
+ * featomic. */
 featomic_status_t featomic_b200_set_contraction_engine(int32_t tensor_cores, int32_t channels_per_round);
 
 /* Kernels of the FP64 spherical expansion (featomic_calculator_compute and

@@ -18,12 +18,15 @@
 // once and read twice.  A direction's terms are evaluated for both atoms of a
 // pair instead; channels with the same knots (all of them, or two groups) share
 // the interval search and the Hermite weights (with seven of each per
-// direction they were a quarter of the instructions and half of the time).  Bound by instruction
-// issue (a third of the slots) and the latency of its load chain.  FP32,
-// lmax 6, nmax 8: 20 000 atoms with 52 directions 0.25 ms (pair records and
-// an expansion kernel: 0.80 ms), 134 128 atoms of molecules 0.94 ms (2.88);
-// FP64 values of 16 600 atoms of molecules 0.39 ms (1.71 with a CTA per
-// segment).
+// direction they were a quarter of the instructions and half of the time).
+// Bound by the latency of its chain of loads and recursions: 20 000 atoms in FP32
+// issue 1.9 of 4 instructions a cycle at 19 warps per SM (96 registers, shared
+// memory), 4.2 of 9 stall cycles an instruction wait for a load.  FP32, lmax 6,
+// nmax 8: 20 000 atoms with 52 directions 0.30 ms (pair records and an expansion
+// kernel: 0.80 ms), 134 128 atoms of molecules 1.02 to 1.12 ms (2.88); FP64 values
+// of 16 600 atoms of molecules 0.36 ms (1.71 with a CTA per segment).  Small bases
+// of many atoms gain least: FP64, 8000 atoms, nmax 4, lmax 3 93 us (71 by pair
+// records).
 //
 // The sums use the operations of pair_features_kernel / se_accumulate_kernel
 // in their order; without FMA contraction the results are bit-identical.

@@ -13,10 +13,12 @@
 //                (l, m, n), segment reduced in registers (no atomics), inverse
 //                pairs with (-1)^l (spherical_expansion_pair.rs:130-163), self
 //                term on l = 0
-//   contraction  warp per centre on the tensor cores (dense_warp.cu); here, for
-//                the CUDA-core engine and larger bases: CTA per centre,
-//                coefficients in shared memory, thread per (species pair
-//                a <= b, l, n1) with a register row over n2:
+//   contraction  warp per centre on the tensor cores (dense_warp.cu), FP32 of
+//                larger bases on tcgen05 (dense_mma.cu); here, for the
+//                CUDA-core engine, larger bases yet, and FP64 where its rule
+//                says so: CTA per centre, coefficients in shared memory,
+//                thread per (species pair a <= b, l, n1) with a register row
+//                over n2:
 //                P[l n1 n2] = sum_m c_a[l m n1] c_b[l m n2] / ((-1)^l sqrt(2l+1)),
 //                times sqrt(2) when a != b (power_spectrum.rs:529-780)
 //

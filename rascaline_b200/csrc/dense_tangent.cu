@@ -9,9 +9,11 @@
 // weights; both then the spline rows and the sums over directions.  Nothing
 // per pair goes to memory, where the general path writes pair records with
 // derivatives and a tangent per (pair, l, m) and reads both again.  Bound by
-// the latency of its load and recursion chains.  FP32, lmax 6, nmax 8: 1500
-// atoms of 3 species 64 us (188 us by pair records); with the power spectrum's
-// tangent 6000 atoms of 4 species 287 us (1033), FP64 533 (1558).
+// the latency of its load and recursion chains: 127 registers and the shared
+// memory leave 14 warps per SM, which issue 1.3 of 4 instructions a cycle.  FP32,
+// lmax 6, nmax 8: 1500 atoms of 3 species 53 to 64 us (188 us by pair records);
+// with the power spectrum's tangent 6000 atoms of 4 species 240 us (1033), FP64
+// 514 (1558).  dense_tangent_by_centre below says where it is used.
 #include "centre_expansion.cuh"
 #include "dense.hpp"
 

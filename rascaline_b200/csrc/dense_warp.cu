@@ -1,5 +1,6 @@
 // Per-centre contractions of the dense power spectrum with a warp per centre,
-// straight from global memory to matrix instructions:
+// straight from global memory to matrix instructions (larger bases in FP32 are in
+// dense_mma.cu):
 //
 //   values  P_l = X_l^T X_l, X_l[m][(s, n)] = c[s][l m][n]
 //           P_ab[l][n1][n2] = scale(l, a != b) P_l[(a, n1), (b, n2)]
@@ -16,8 +17,9 @@
 // with operands split into hi + lo, three products; FP64: m8n8k4) is the
 // layout of the coefficients in memory: a fragment of X_l is four rows m of
 // eight consecutive (s, n), one coalesced load per element, and is the left
-// and the right operand of P_l at once.  Both kernels are bound by their HBM
-// streams.
+// and the right operand of P_l at once.  The kernels are bound by the latency of
+// those loads: a warp's steps follow one another, at a third of the warps that an
+// SM holds (65 to 128 registers).
 #include <algorithm>
 #include <type_traits>
 
@@ -116,10 +118,11 @@ __device__ __forceinline__ void step_upper2(double (&acc)[NT][NT][2], const doub
 
 // nmax <= 8 and NT <= 4 species: a tile is one species pair (nmax < 8 padded
 // with zeros), and everything that depends on the species is known to the
-// compiler.  Bound by instruction issue rather than memory: 20 000 atoms, 4
+// compiler.  Bound by load latency (10 of 15 stall cycles an instruction at 21
+// warps per SM, DRAM half busy, 1.4 of 4 instructions a cycle): 20 000 atoms, 4
 // species, lmax 6, nmax 8 (125 MB read, 358 written) 0.109 ms = 4.4 TB/s, 0.232
-// with four centres on a tcgen05 tile; with the species found at run time
-// (below) 0.174.  FP64, 2000 atoms: 17 us, 52 with a CTA per centre.
+// with four centres on a tcgen05 tile; with the species found at run time 0.174.
+// FP64, 2000 atoms: 17 us, 52 with a CTA per centre.
 // `energy`: with a linear model's weights [species][keys][props], the centre's
 // energy sum_P w P from the values on their way out (134 128 atoms: 0.72 ms;
 // 1.49 + 0.53 with a kernel that read them back): a lane's ten products of an l
@@ -365,8 +368,9 @@ __global__ void __launch_bounds__(32 * DW_WARPS, 2) dense_contraction_warp(Dense
 // by 8 x 8 tiles over (a; eight m), with the scale of the species pair in the
 // right operand.  MMA slot k = t of the two steps of a species is q = 2 t and
 // 2 t + 1.  Bound by the loads of G (read once straight and once transposed):
-// 2000 atoms, 4 species, lmax 6: 37 us, 98 with a CTA per centre and
-// its rows staged in shared memory.
+// L1 77 % busy, 12 of 17 stall cycles an instruction wait for a load (4000
+// atoms).  2000 atoms, 4 species, lmax 6: 37 us, 98 with a CTA per centre and its
+// rows staged in shared memory.
 template <int NT, bool N8>
 __global__ void __launch_bounds__(32 * DW_WARPS, 2) dense_grad_coef_tiles(DenseArgs<double> a) {
     __shared__ double scales[64];
@@ -430,8 +434,10 @@ __global__ void __launch_bounds__(32 * DW_WARPS, 2) dense_grad_coef_tiles(DenseA
 // 32, split into hi and lo) is built in shared memory and kept in each warp's
 // registers, and the warps take the columns (c, m), eight at a time.  MMA
 // slots k = t and t + 4 are (b, q) = 2 t and 2 t + 1, so that both operands
-// are read in pairs.  134 128 atoms, 4 species, lmax 6, nmax 8 (841 MB read
-// and written): 0.74 ms; 2.95 with an operand per centre on tcgen05 tiles.
+// are read in pairs.  Bound by load latency and its 116 registers (15 warps per
+// SM, 1.7 of 4 instructions a cycle, DRAM a quarter busy).  134 128 atoms, 4
+// species, lmax 6, nmax 8 (841 MB read and written): 0.74 to 0.83 ms; 2.95 with an
+// operand per centre on tcgen05 tiles.
 constexpr int DG_CENTRES = 64;
 constexpr int DG_PITCH = 40;  // floats; rows 4 g apart hit banks 8 bytes apart
 

@@ -547,8 +547,9 @@ __global__ void __launch_bounds__(128) se_output_rows_kernel(SeOutArgs a, int do
 // positions gradient rows (spherical_expansion.rs:468-521): for every
 // neighbour entry of a centre (and the centre itself) the rows of all l at
 // once, from the pairs' gradients (or the centre's own).  SE_SPLIT CTAs share
-// a centre's entries.  Bound by the memory stream: a row set is 3 (l m n)
-// doubles read and written.  Row numbers come from the neighbourhood tables
+// a centre's entries.  Bound by the latency of reading a row set of 3 (l m n)
+// doubles before it is written (11 of 16 stall cycles an instruction, DRAM 45 %
+// busy).  Row numbers come from the neighbourhood tables
 // on the device: the list of rows that the host used to make and upload (7
 // per entry) was 6 of the 7.3 ms of a call on 500 atoms (1.4 now), and one CTA
 // per row of 24 to 312 doubles took 358 us where this takes 165 (340 MB

@@ -2,10 +2,10 @@
 // on the GPU.  For every periodic system:
 //
 //   host    k-vectors of the cell inside the k_cutoff ball (one of each +-k
-//           pair), the density's Fourier transform f(k) and the radial
-//           integral R_nl(|k|) (spline or analytic) per k-vector
-//   kernel  lode_projection_kernel: T[k][(l m n)] = R_nl(|k|) Y_lm(k^), the
-//           even l first, then the odd l
+//           pair) and the density's Fourier transform f(k); the radial integral
+//           R_nl(|k|) per k-vector where it is analytic
+//   kernel  lode_projection_kernel: R_nl(|k|) from its spline, T[k][(l m n)] =
+//           R_nl(|k|) Y_lm(k^), the even l first, then the odd l
 //   kernel  lode_phases_kernel: cos(k.r_i), sin(k.r_i) for every atom and k
 //   kernel  lode_type_sums_kernel: the same summed over the atoms of each type
 //   kernel  lode_gemm_kernel: values (rows: centre i towards neighbour type t)
@@ -15,9 +15,10 @@
 //           factor of (i, j), times 4 pi / V f(k), made on the way into
 //           shared memory
 //
-// The sums over k run in featomic's order inside each split of the k-vectors
-// (the sign (-1)^{l/2}, (-1)^{(l+1)/2} applied at the end, which is exact),
-// then the central-atom and k = 0 terms in featomic's order.
+// The sums over k run by fours (a tensor-core step) inside each split of the
+// k-vectors, then over the splits: not featomic's order, and the same from call
+// to call.  The sign (-1)^{l/2}, (-1)^{(l+1)/2} is applied at the end, which is
+// exact, then the central-atom and k = 0 terms in featomic's order.
 #include <algorithm>
 #include <chrono>
 #include <cmath>
@@ -531,7 +532,8 @@ __device__ __forceinline__ void lode_cp16(void* dst, const void* src, bool valid
 // rows of the left operand are built from cos and sin (loaded one step ahead
 // into registers) and stored to shared memory, T's rows arrive by cp.async in
 // two buffers.  Bound by the FP64 tensor pipe (2 x rows x k x columns flops;
-// about 36 TFLOP/s); 64 rows keep the reads of T and of cos / sin, both from
+// about 36 TFLOP/s; the longest stall is the pipe's throttle, 3.7 of 13 cycles an
+// instruction); 64 rows keep the reads of T and of cos / sin, both from
 // L2, below it, and 128 registers (four CTAs per SM) hide the two barriers of
 // a step.  Values of 1000 atoms, 3 types, 4522 k-vectors and 392 coefficients
 // (10.6 GFLOP): 0.51 ms = 20.7 TFLOP/s; 0.68 ms with three CTAs per SM and
