@@ -19,10 +19,11 @@ from rascaline_b200 import torch_api  # noqa: E402
 
 
 def _product(l1, l2, lam):
+    # enough samples for the tensor-core kernel
     generator = torch.Generator().manual_seed(l1)
-    a = torch.randn((2, 2 * l1 + 1, 20), generator=generator, dtype=torch.float64).cuda()
-    b = torch.randn((2, 2 * l2 + 1, 20), generator=generator, dtype=torch.float64).cuda()
-    out = torch.empty((2, 2 * lam + 1, 400), dtype=torch.float64, device="cuda")
+    a = torch.randn((2000, 2 * l1 + 1, 20), generator=generator, dtype=torch.float64).cuda()
+    b = torch.randn((2000, 2 * l2 + 1, 20), generator=generator, dtype=torch.float64).cuda()
+    out = torch.empty((2000, 2 * lam + 1, 400), dtype=torch.float64, device="cuda")
 
     def call():
         cg.cg_tensor_products([(a, b, out, lam)])
